@@ -7,6 +7,9 @@
 
 namespace {
 
+// Ranges per kv head that run at once in long contexts (0: the heads alone are more).
+int ranges_at_once(int n_kv, int sms) { return 2 * sms / n_kv; }
+
 template <bool FUSED, bool EXT = false>
 int launch_decode_mma(void* out, long long out_stride, const void* q, long long q_stride, const void* k_pages,
                       const void* v_pages, const int* block_table, int table_width, const int* kv_lens,
@@ -16,7 +19,7 @@ int launch_decode_mma(void* out, long long out_stride, const void* q, long long 
   dim3 grid(splits, n_kv, n_entries);
   const float scale_log2e = EXT ? scale : scale * 1.4426950408889634f;
   const int group_rows = n_heads / n_kv < decode_mma::ROWS ? n_heads / n_kv : decode_mma::ROWS;
-  // 2 to 8 ranges whose shares fit the first CTA's receive buffer, and a grid of at most two
+  // 2 to 8 ranges, a receive buffer that holds each CTA's part of the outputs, and a grid of at most two
   // waves: merge inside a cluster, no scratch.  (Measured at 64 requests, 512 CTAs: 30 us with
   // clusters against 23 us with the counter-based merge; at 8 requests 9.3 us against 13.5 us.)
   constexpr int RECV_LIMIT = 64 * 1024;
@@ -33,20 +36,28 @@ int launch_decode_mma(void* out, long long out_stride, const void* q, long long 
   // with one stage, which at head size 64 is also held to 128 registers so that four CTAs share
   // an SM and the grid still runs as one wave where it can (128 requests x 4 kv heads at 640
   // keys: 22.9 us against 28.0 us).
-  const long long ctas = (long long)splits * n_kv * n_entries;
+  // long contexts: about two ranges per SM over all requests (range_length), of a grid that has room for more
+  const int balance = !cluster && max_keys > 2048 ? ranges_at_once(n_kv, llmk_sm_count()) : 0;
+  // (as many CTAs as there can be ranges, see range_length: one wave, or the even share's)
+  if (balance > 0) grid = dim3((unsigned)((long long)splits * n_entries < balance + n_entries ? splits * n_entries : balance + n_entries), n_kv, 1);
+  long long ctas = (long long)splits * n_kv * n_entries;
+  if (balance > 0 && ctas > (long long)(balance > n_entries ? balance : n_entries) * n_kv)
+    ctas = (long long)(balance > n_entries ? balance : n_entries) * n_kv;
   const bool light = !cluster && ctas > (long long)(head_dim == 64 ? 2 : 1) * llmk_sm_count();
-  // long contexts: about two ranges per SM over all requests (see the kernel)
-  const int balance = !cluster && max_keys > 2048 ? (2 * llmk_sm_count() + n_kv - 1) / n_kv : 0;
   // per warp its stages of a tile of keys and a tile of values: NST in the kernel
   const int stage_bytes = 4 * ((cluster || light) ? 1 : head_dim == 64 ? 3 : 2) * 2 * decode_mma::TILE * head_dim * 2;
-  using Kernel = decltype(&decode_mma::decode_attention_mma_kernel<64, false, FUSED, false, EXT>);
-  const Kernel kern = head_dim == 64
-      ? (cluster ? decode_mma::decode_attention_mma_kernel<64, true, FUSED, false, EXT>
-                 : light ? decode_mma::decode_attention_mma_kernel<64, false, FUSED, true, EXT> : decode_mma::decode_attention_mma_kernel<64, false, FUSED, false, EXT>)
-      : (cluster ? decode_mma::decode_attention_mma_kernel<128, true, FUSED, false, EXT>
-                 : light ? decode_mma::decode_attention_mma_kernel<128, false, FUSED, true, EXT> : decode_mma::decode_attention_mma_kernel<128, false, FUSED, false, EXT>);
-  static bool configured[2][3] = {{false, false, false}, {false, false, false}};
-  const int variant = cluster ? 1 : light ? 2 : 0;
+  using namespace decode_mma;
+  using Kernel = decltype(&decode_attention_mma_kernel<64, false, FUSED, false, EXT>);
+  static const Kernel kernels[2][5] = {
+      {decode_attention_mma_kernel<64, false, FUSED, false, EXT>, decode_attention_mma_kernel<64, true, FUSED, false, EXT>,
+       decode_attention_mma_kernel<64, false, FUSED, true, EXT>, decode_attention_mma_kernel<64, false, FUSED, false, EXT, true>,
+       decode_attention_mma_kernel<64, false, FUSED, true, EXT, true>},
+      {decode_attention_mma_kernel<128, false, FUSED, false, EXT>, decode_attention_mma_kernel<128, true, FUSED, false, EXT>,
+       decode_attention_mma_kernel<128, false, FUSED, true, EXT>, decode_attention_mma_kernel<128, false, FUSED, false, EXT, true>,
+       decode_attention_mma_kernel<128, false, FUSED, true, EXT, true>}};
+  static bool configured[2][5] = {};
+  const int variant = cluster ? 1 : (light ? 2 : 0) + (balance > 0 ? (light ? 2 : 3) : 0);
+  const Kernel kern = kernels[head_dim == 128][variant];
   if (!configured[head_dim == 128][variant]) {
     cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, stage_bytes + (cluster ? RECV_LIMIT : 0));
     if (err != cudaSuccess) return llmk_fail((int)err, "attention_decode: cannot set the shared memory size: %s", cudaGetErrorString(err));
@@ -68,17 +79,35 @@ int launch_decode_mma(void* out, long long out_stride, const void* q, long long 
     cfg.attrs = attr;
     cfg.numAttrs = llmk_pdl_enabled() ? 2 : 1;
     cudaLaunchKernelEx(&cfg, kern, (__nv_bfloat16*)out, out_stride, scratch, (const __nv_bfloat16*)q, q_stride,
-                       (__nv_bfloat16*)k_pages, (__nv_bfloat16*)v_pages, block_table, table_width, kv_lens, n_heads,
+                       (__nv_bfloat16*)k_pages, (__nv_bfloat16*)v_pages, block_table, table_width, kv_lens, n_entries, n_heads,
                        n_kv, page_size, window, scale_log2e, splits, fused, kv_share, opt, balance);
   } else {
     launch_kernel(kern, grid, dim3(decode_mma::THREADS), (size_t)stage_bytes, stream, (__nv_bfloat16*)out, out_stride, scratch,
                   (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)k_pages, (__nv_bfloat16*)v_pages, block_table,
-                  table_width, kv_lens, n_heads, n_kv, page_size, window, scale_log2e, splits, fused, kv_share, opt, balance);
+                  table_width, kv_lens, n_entries, n_heads, n_kv, page_size, window, scale_log2e, splits, fused, kv_share, opt, balance);
   }
   LLMK_LAUNCH_CHECK("attention_decode_mma");
 }
 
 }  // namespace
+
+// The ranges that the kernel gives n_entries requests of these lengths (host arrays) on a GPU of `sms` SMs, as a launch with `splits` ranges
+// a request in its grid does; returns their number, over all kv heads.
+LLMK_API int llmk_decode_attention_ranges(const int* kv_lens, int n_entries, int n_kv, int window, int chunk, int keep_first, int splits,
+                                          int sms, int* ranges) {
+  using namespace decode_mma;
+  const Mask mask{window, chunk, keep_first};
+  int running = 0;
+  auto over = [&](auto&& count) {
+    int sum = 0;
+    for (int i = 0; i < n_entries; ++i) sum += count(mask.visible(kv_lens[i]));
+    return sum;
+  };
+  LLMK_REQUIRE(n_entries > 0 && n_kv > 0 && splits > 0 && ranges_at_once(n_kv, sms) > 0, "decode_attention_ranges: bad sizes");
+  const int length = range_length(over, splits, ranges_at_once(n_kv, sms), running);
+  for (int i = 0; i < n_entries; ++i) ranges[i] = ranges_of(mask.visible(kv_lens[i]), length, splits);
+  return running * n_kv;
+}
 
 // Whether llmk_paged_attention_decode_mma takes these sizes: bfloat16 with a head size of 64 or
 // 128, pages of a power of two, rows of q that start on 4-byte boundaries.

@@ -1,8 +1,8 @@
 // Decode attention on the warp-level tensor cores (bfloat16, head size 64 or 128).
 //
-// The same split of the keys into ranges, one CTA per (range, kv head, request), and the same
-// merge by the last CTA as the CUDA-core kernel in attention_decode.cu; what differs is the
-// inside of a range.  The query heads of the kv group are the rows of an m16n8k16 MMA (up to 16
+// The same split of the keys into ranges, one CTA per (range, kv head, request), as the CUDA-core
+// kernel in attention_decode.cu, merged by the last CTA to arrive as there or, few short ranges, by a
+// cluster's CTAs a part each; what differs most is the inside of a range.  The query heads of the kv group are the rows of an m16n8k16 MMA (up to 16
 // per pass): one instruction scores 8 keys for all of them, so the arithmetic per key no longer
 // grows with the group size.  Each of the four warps works alone on tiles of 32 keys, without
 // block-wide barriers: keys and values are staged per warp through one to three stages of shared
@@ -107,6 +107,9 @@ __device__ __forceinline__ float2 sum2(const MaybePartial<__nv_bfloat16>& s, siz
 // memory, no fence, no counter.  Every CTA arrives at a first cluster barrier when it starts and waits for it only
 // before it writes to the others, which must be running by then; a second barrier publishes the writes.
 //
+// BALANCE: long contexts, whose ranges are handed out by the requests' lengths (range_length).  A variant of its own, because the code alone,
+// never run, cost short contexts 0.7 us a launch (64 requests of 600 keys inside a decode step).
+//
 // FUSED: the kernel takes the row of the QKV product itself (a tensor or unsummed split-K
 // partial results) instead of rotated queries.  Every CTA sums and rotates its group's queries
 // into shared memory; the CTA whose range holds the newest position also sums and rotates that
@@ -141,13 +144,64 @@ struct Options {
   const float* sigmoid_bias;     // weights sigmoid(score + bias[head]), nothing is normalised
 };
 
-template <int HS, bool CLUSTER, bool FUSED, bool LIGHT = false, bool EXT = false>
+// Which of a request's keys its newest token sees: a window's (0: all) or a chunk's, and the first ones that a window keeps.
+struct Mask {
+  int window, chunk, keep_first;
+  __host__ __device__ int begin(int held) const {
+    const int pos = held - 1;
+    return chunk > 0 ? pos / chunk * chunk : (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
+  }
+  __host__ __device__ int kept(int begin) const { return keep_first < begin ? keep_first : begin; }
+  __host__ __device__ int visible(int held) const { return held > 0 ? held - begin(held) + kept(begin(held)) : 0; }
+};
+
+// How long contexts are cut: `balance` ranges for all requests together and kv head, as many as run at once, handed out by length, so that
+// one long request among short ones is not walked by as few CTAs as each of them (one of 6,000 keys beside seven of 400, 8 kv heads of
+// 128: four ranges a request 33 us a launch, by length 14.7 us).  All requests get ranges of about one length, the shortest with which they
+// run in one wave.  (Shares rounded to the nearest gave equal requests a piece more than fits: 8 of 8,192 keys, 37 places taken as 5 each, 320
+// CTAs for 296 places, 69 us; 4 each 49 us.  8 of 3,000 33.9 -> 24.5 us; at head size 64, 4 kv heads, 8 of 8,192 24.0 -> 20.6, 10 of 8,192 29.1 ->
+// 24.1, 6,000 beside 400 12.7 -> 10.4; slower: 12 of 300 to 3,600 keys 24.2 -> 25.8, 48 of 4,096 at head size 64 42.5 -> 45.6, where more than one
+// wave of short ranges keeps more bytes in flight.)  Where that length would pass twice the even share, a few long requests are among many
+// short ones, whose places are soon free again, and the even share is taken.  `over` sums a function of the visible keys over the requests;
+// at most `splits` ranges a request; running: the ranges of all of them, at most `balance` plus the number of requests.
+__host__ __device__ inline int ranges_of(int keys, int length, int splits) {
+  const int n = (keys + length - 1) / length;
+  return n < 1 ? 1 : n < splits ? n : splits;      // (an entry without keys: zeros are written)
+}
+template <typename Over>
+__host__ __device__ inline int range_length(Over&& over, int splits, int balance, int& running) {
+  // length 0: the sum of the keys; then the even share, twice that, and by halves to 3 % of it between the two.  (One place that walks the
+  // entries: a launch runs through this code once, so that fetching it is what it costs.)
+  int length = 0, even = 0, fewest = 0, below = 0, fit = 0, at_once = 0;
+  while (true) {
+    const int sum = over([&](int n) { return length ? ranges_of(n, length, splits) : n; });
+    const bool fits = sum <= balance;
+    if (length == 0) {
+      const int share = (sum + balance - 1) / balance;
+      length = even = share > 256 ? share : 256;
+      continue;
+    }
+    if (below == 0) {                                   // the even share
+      if (fits) { running = sum; return even; }
+      fewest = sum;
+      below = even;
+      length = 2 * even;
+      continue;
+    }
+    if (fits) { fit = length; at_once = sum; } else { below = length; }
+    if (fit == 0) { running = fewest; return even; }
+    if ((fit - below) * 32 < even) { running = at_once; return fit; }
+    length = (fit + below) / 2;
+  }
+}
+
+template <int HS, bool CLUSTER, bool FUSED, bool LIGHT = false, bool EXT = false, bool BALANCE = false>
 __global__ void __launch_bounds__(THREADS, (LIGHT && HS == 64) ? 4 : 1)
 decode_attention_mma_kernel(__nv_bfloat16* __restrict__ out, long long out_stride, float* __restrict__ scratch,
                             const __nv_bfloat16* __restrict__ q, long long q_stride,
                             __nv_bfloat16* __restrict__ k_pages, __nv_bfloat16* __restrict__ v_pages,
                             const int* __restrict__ block_table, int table_width, const int* __restrict__ kv_lens,
-                            int n_heads, int n_kv, int page_size, int window, float scale_log2e, int splits,
+                            int n_entries, int n_heads, int n_kv, int page_size, int window, float scale_log2e, int splits,
                             FusedQkv fused, int kv_share, Options opt, int balance) {
   static_assert(!(FUSED && EXT), "the fused kernel has no options");
   constexpr float LOG2E = 1.4426950408889634f;
@@ -176,8 +230,42 @@ decode_attention_mma_kernel(__nv_bfloat16* __restrict__ out, long long out_strid
   float* recv_s = reinterpret_cast<float*>(vbuf + 4 * WARP_BYTES);   // CLUSTER: what the ranges send to this CTA
   pdl_launch_dependents();
   if (CLUSTER) tc::cluster_arrive();
-  const int split = blockIdx.x, g = blockIdx.y, e = blockIdx.z;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = blockIdx.y;
+  const Mask mask{window, EXT ? opt.chunk : 0, EXT ? opt.keep_first : 0};
+  // The entry, its range and how many it has: the grid's, or (BALANCE) by the requests' lengths, the ranges of all entries one after
+  // the other along blockIdx.x.  Every CTA finds that from the lengths, warp by warp, before it waits for anybody.  (Grids of `splits` places
+  // an entry, of which the unneeded ones leave at once, leave the SMs unevenly filled: 8 requests of 8,192 keys, 8 kv heads of 128, 4 of 16
+  // places each in use, 57 us, and packed 49 us.)
+  int e = blockIdx.z, split = blockIdx.x, n_ranges = splits;
+  int running = (int)(gridDim.x * gridDim.z);                 // ranges of all entries, per kv head
+  if constexpr (BALANCE) {
+    auto seen_by = [&](int i) { return mask.visible(min(kv_lens[i], table_width * page_size)); };
+    auto over_entries = [&](auto&& count) {
+      int sum = 0;
+#pragma unroll 1
+      for (int i = lane; i < n_entries; i += 32) sum += count(seen_by(i));
+      return __reduce_add_sync(0xffffffffu, sum);
+    };
+    const int length = range_length(over_entries, splits, balance, running);
+    e = -1;
+#pragma unroll 1
+    for (int i0 = 0, before = 0; i0 < n_entries && e < 0; i0 += 32) {
+      const int own = i0 + lane < n_entries ? ranges_of(seen_by(i0 + lane), length, splits) : 0;
+      int upto = own;
+#pragma unroll
+      for (int o = 1; o < 32; o *= 2) {
+        const int below = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += below;
+      }
+      const uint32_t behind = __ballot_sync(0xffffffffu, (int)blockIdx.x < before + upto);
+      const int at = behind ? __ffs(behind) - 1 : 31;
+      const int first = before + __shfl_sync(0xffffffffu, upto - own, at);
+      n_ranges = __shfl_sync(0xffffffffu, own, at);
+      if (behind) { e = i0 + at; split = (int)blockIdx.x - first; }
+      before = first + n_ranges;
+    }
+    if (e < 0) return;                                        // the grid holds the most ranges that there can be
+  }
   const int group = n_heads / n_kv;
   // kv_share > 1: that many neighbouring groups of query heads read one key/value head (a group of many heads split over
   // several CTAs, each with its own pass over the keys): the pages hold n_kv / kv_share heads
@@ -194,27 +282,13 @@ decode_attention_mma_kernel(__nv_bfloat16* __restrict__ out, long long out_strid
     return;
   }
   const int pos = n_held - 1;
-  const int lo = EXT && opt.chunk > 0 ? pos / opt.chunk * opt.chunk : (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
+  const int lo = mask.begin(n_held);
   // EXT: the visible keys as a list, [0, keep_end) and then [lo, pos]; below, a key's number is its place in that list and
   // `last` the newest key's.  Otherwise a key's number is its position.
-  const int keep_end = EXT ? min(opt.keep_first, lo) : 0, skip = EXT ? lo - keep_end : 0;
+  const int keep_end = mask.kept(lo), skip = EXT ? lo - keep_end : 0;
   const int first = EXT ? 0 : lo, last = pos - skip;
   const int n_keys = last - first + 1;
   auto position_of = [&](int k) { return EXT && k >= keep_end ? k + skip : k; };
-  // Ranges of this request.  balance > 0 (long contexts): about so many for all requests together and kv head, handed out by length, so
-  // that one long request among short ones is not walked by as few CTAs as each of them (one of 6,000 keys beside seven of 400, 8 kv
-  // heads of 128: four ranges a request 40 us a launch, by length 18 us).  Every CTA sums the lengths, warp by warp, before it
-  // waits for anybody; the grid holds `splits` ranges a request, and those that a request does not need leave.
-  int n_ranges = splits;
-  if (!CLUSTER && balance > 0) {
-    int total = 0;
-    for (int i = lane; i < (int)gridDim.z; i += 32) {
-      const int held = min(kv_lens[i], table_width * page_size);
-      total += window > 0 ? min(held, window) : max(held, 0);
-    }
-    total = __reduce_add_sync(0xffffffffu, total);
-    n_ranges = min(min(splits, (n_keys + 255) / 256), max(1, (int)((float)n_keys * (float)balance / (float)total + 0.5f)));
-  }
   int chunk = (n_keys + n_ranges - 1) / n_ranges;
   chunk = (chunk + TILE - 1) / TILE * TILE;
   const int n_active = min(splits, (n_keys + chunk - 1) / chunk);      // ranges that hold keys
@@ -278,10 +352,10 @@ decode_attention_mma_kernel(__nv_bfloat16* __restrict__ out, long long out_strid
   for (int j = 0; j < NST; ++j)
     if (j < n_tiles) stage_tile(j);
   {
-    // at most 32 MB over the whole grid: asking for more than L2 keeps evicts the lines before
+    // at most 32 MB over all ranges that run: asking for more than L2 keeps evicts the lines before
     // they are used and fetches them from memory twice (long ranges stream through the stages)
     constexpr int LINES = HS * 2 / 128;                    // 128-byte lines per row
-    const int ask_limit = (32 << 20) / (int)(gridDim.x * gridDim.y * gridDim.z) / (HS * 4);
+    const int ask_limit = (32 << 20) / (running * (int)gridDim.y) / (HS * 4);
     const int n_rows = min(ask_limit, max(0, k_end - k_begin - NST * 4 * TILE));
     for (int i = tid; i < n_rows * LINES * 2; i += THREADS) {
       const int which = i & 1, line = (i >> 1) % LINES, kp = k_begin + NST * 4 * TILE + (i >> 1) / LINES;
@@ -327,7 +401,7 @@ decode_attention_mma_kernel(__nv_bfloat16* __restrict__ out, long long out_strid
 
   int* counters = reinterpret_cast<int*>(scratch);
   float* partial_ml = scratch + COUNTER_WORDS;
-  float* partial_o = partial_ml + (size_t)gridDim.z * n_heads * splits * 2;
+  float* partial_o = partial_ml + (size_t)n_entries * n_heads * splits * 2;
 
   // (in a cluster a range without keys still has to meet the others at the barriers)
   for (int h0 = 0; h0 < group && (CLUSTER || k_begin < k_end); h0 += ROWS) {

@@ -1434,8 +1434,8 @@ def decode_splits(n_entries: int, n_kv: int, max_keys: int, sms: int = 0) -> int
 
 
 def decode_places(n_entries: int, n_kv: int, max_keys: int, sms: int = 0) -> int:
-    """Ranges per request that the grid of the tensor-core decode kernel holds.  Beyond 2,048 keys the kernel hands the ranges out by
-    the requests' lengths (a launch must not depend on them), so the grid has room for one request with four times its share."""
+    """The most ranges that the tensor-core decode kernel gives one request.  Beyond 2,048 keys it hands the ranges out by the requests'
+    lengths (a launch must not depend on them): room for one request with four times its share."""
     s = decode_splits(n_entries, n_kv, max_keys, sms)
     return s if max_keys <= 2048 else max(s, min(64, 4 * s, max_keys // 256))
 
