@@ -137,13 +137,23 @@ namespace {
 // VEC: four channels at a time (dim and the rows on the 4-grid).  A few tokens are bound by the loads of their partial results (eight
 // of a channel, a round trip to L2 for every four), so a CTA of 512 threads has a row of 2,560 channels in flight at once, and the angles
 // are made once per CTA: 8 tokens, 20 heads of 128, 18.9 -> 8.3 us a launch inside a decode step.
+// Shared memory: the row, rounded up to whole pairs of floats, then a cosine and a sine per pair that turns (`table`), unless a row
+// and angles of that size do not fit together: every pair then makes its own.
+constexpr size_t NORM_ROPE_SMEM = 226 * 1024;      // of the 227 KB of a CTA; the sums' scratch takes 128 bytes
+__host__ __device__ inline size_t norm_rope_row_floats(int channels) { return ((size_t)channels + 1) / 2 * 2; }
+size_t norm_rope_smem(int channels, int rot_pairs, bool& table) {
+  const size_t row = norm_rope_row_floats(channels) * sizeof(float), both = row + (size_t)rot_pairs * sizeof(float2);
+  table = both <= NORM_ROPE_SMEM;
+  return table ? both : row;
+}
+
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(512)
 norm_rope_kv_write_kernel(MaybePartial<T> src, long long src_stride, T* __restrict__ q_out, long long q_out_stride,
                           const float* __restrict__ q_gain, const float* __restrict__ k_gain, float eps,
                           const float* __restrict__ freqs, int rot_pairs, int halves, const int* __restrict__ positions,
                           const int* __restrict__ slot_map, T* __restrict__ k_pages, T* __restrict__ v_pages,
-                          int n_heads, int n_kv, int dim, int vdim, int page_size, float amp, int v_from_k) {
+                          int n_heads, int n_kv, int dim, int vdim, int page_size, float amp, int v_from_k, int table) {
   extern __shared__ float row_s[];            // [(n_heads + n_kv) * dim]
   __shared__ float red[32];
   pdl_launch_dependents();
@@ -153,12 +163,14 @@ norm_rope_kv_write_kernel(MaybePartial<T> src, long long src_stride, T* __restri
   const size_t row = (size_t)t * src_stride;
   const int qn = n_heads * dim, kn = n_kv * dim;
   float sq = 0.f, sk = 0.f;
-  float2* turn_s = reinterpret_cast<float2*>(row_s + ((qn + kn) + 1) / 2 * 2);      // [rot_pairs]: cosine, sine
-  for (int i = threadIdx.x; i < rot_pairs; i += blockDim.x) {
+  auto turn = [&](int i) {
     float sn, cs;
     sincosf(pos * freqs[i], &sn, &cs);
-    turn_s[i] = make_float2(cs * amp, sn * amp);
-  }
+    return make_float2(cs * amp, sn * amp);
+  };
+  float2* turn_s = reinterpret_cast<float2*>(row_s + norm_rope_row_floats(qn + kn));      // [rot_pairs]: cosine, sine
+  if (table)
+    for (int i = threadIdx.x; i < rot_pairs; i += blockDim.x) turn_s[i] = turn(i);
   size_t k_base = 0, v_base = 0;
   if (n_kv) {
     const int slot = slot_map[t];
@@ -203,7 +215,7 @@ norm_rope_kv_write_kernel(MaybePartial<T> src, long long src_stride, T* __restri
       const int d0 = halves ? i : 2 * i, d1 = halves ? i + rot_pairs : 2 * i + 1;
       const float a = row_s[c_base + d0] * r * (gain ? gain[g_base + d0] : 1.f);
       const float b = row_s[c_base + d1] * r * (gain ? gain[g_base + d1] : 1.f);
-      const float2 cs = turn_s[i];
+      const float2 cs = table ? turn_s[i] : turn(i);
       dst[d0] = from_f32<T>(a * cs.x - b * cs.y);
       dst[d1] = from_f32<T>(b * cs.x + a * cs.y);
     } else {
@@ -401,6 +413,14 @@ LLMK_API int llmk_rope_pairs_kv_write(const void* qkv, const float* partials, in
   });
 }
 
+// The dynamic shared memory that llmk_norm_rope_kv_write asks for with gains, and (row_bytes) where in it the angles begin.
+LLMK_API long long llmk_norm_rope_smem(int channels, int rot_pairs, long long* row_bytes) {
+  bool table;
+  const size_t bytes = norm_rope_smem(channels, rot_pairs, table);
+  *row_bytes = (long long)(norm_rope_row_floats(channels) * sizeof(float));
+  return (long long)bytes;
+}
+
 // As llmk_rope_pairs_kv_write, with the RMS norm of the whole q and k projections first (gains float32 [n_heads * dim] and
 // [n_kv * dim], each may be null) and the choice of the pairs: halves != 0 turns channel i against i + rot_pairs.  v_from_k: a row
 // is n_heads * dim | n_kv * dim numbers and the values stored are the keys before norm and rotation.
@@ -415,7 +435,8 @@ LLMK_API int llmk_norm_rope_kv_write(const void* qkv, const float* partials, int
   LLMK_REQUIRE(rot_pairs >= 0 && 2 * rot_pairs <= dim, "norm_rope_kv_write: %d pairs do not fit a head of %d", rot_pairs, dim);
   LLMK_REQUIRE(rot_pairs == 0 || freqs != nullptr, "norm_rope_kv_write: frequencies are missing");
   LLMK_REQUIRE(!v_from_k || vdim == dim, "norm_rope_kv_write: keys that are values have one size, not %d and %d", dim, vdim);
-  const size_t smem = (size_t)(n_heads + n_kv) * dim * sizeof(float) + (size_t)rot_pairs * sizeof(float2);
+  bool table;
+  const size_t smem = norm_rope_smem((n_heads + n_kv) * dim, rot_pairs, table);
   LLMK_REQUIRE((size_t)(n_heads + n_kv) * dim * sizeof(float) <= 200 * 1024 || (!q_gain && !k_gain), "norm_rope_kv_write: a projection of %d numbers does not fit shared memory", (n_heads + n_kv) * dim);
   return dispatch_dtype(dtype, [&](auto* tag) {
     using T = LLMK_ELEM(tag);
@@ -425,15 +446,14 @@ LLMK_API int llmk_norm_rope_kv_write(const void* qkv, const float* partials, int
                            n_tokens, n_heads, n_kv, dim, vdim, page_size, amp, v_from_k, stream);
       LLMK_LAUNCH_CHECK("rope_kv_store");
     }
-    if (smem > 48 * 1024)
-    {
+    if (smem > 48 * 1024) {
       cudaFuncSetAttribute(norm_rope_kv_write_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       cudaFuncSetAttribute(norm_rope_kv_write_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     }
     const bool vec = dim % 4 == 0 && src_stride % 4 == 0 && src.vector_ok();
     launch_kernel(vec ? norm_rope_kv_write_kernel<T, true> : norm_rope_kv_write_kernel<T, false>, dim3(n_tokens), dim3(n_tokens <= 128 ? 512 : 256),
                   smem, stream, src, src_stride, (T*)q_out, q_out_stride, q_gain, k_gain, eps, freqs, rot_pairs, halves, positions, slot_map, (T*)k_pages, (T*)v_pages,
-                  n_heads, n_kv, dim, vdim, page_size, amp, v_from_k);
+                  n_heads, n_kv, dim, vdim, page_size, amp, v_from_k, (int)table);
     LLMK_LAUNCH_CHECK("norm_rope_kv_write");
   });
 }
