@@ -1649,9 +1649,9 @@ def paged_attention(out, qkv, k_pages, v_pages, group, ctx, n_heads: int, n_kv: 
     extended = bool(not same or softcap or sink or keep_first or with_dist or with_chunk)
     if (extended and same and ctx.decode_only and qkv.dtype == torch.bfloat16 and head_dim % 16 == 0 and head_dim <= 256
             and not (with_dist and (with_chunk or not ATTENTION_FAST_OPTIONS))
-            and (decode_mma_takes(qkv, head_dim, k_pages.shape[2]) or not with_chunk)):
+            and (not with_chunk or (decode_mma_takes(qkv, head_dim, k_pages.shape[2]) and ctx.n_entries * n_kv <= _ATTN_COUNTER_WORDS))):
         # single tokens: split along the keys, on warp-level MMAs where these take the sizes (the only ones of the two kernels
-        # that know chunks and sigmoid weights)
+        # that know chunks and sigmoid weights; more (request, kv head) pairs of these than there are arrival counters go on below)
         max_keys = min(ctx.kv_bucket or 1 << 30, group.block_table.shape[1] * k_pages.shape[2])
         if with_chunk:                             # as the general kernel is called below: no sink, no kept keys
             sink, sink_values, keep_first = False, None, 0

@@ -74,3 +74,26 @@ def test_chunks_and_sigmoid_weights_are_refused_where_only_the_cuda_core_kernel_
     with pytest.raises(ops.KernelError):
         ops.paged_attention_decode(torch.zeros_like(q), q, kp, kp, torch.zeros(1, 1, dtype=torch.int32, device=DEV),
                                    torch.ones(1, dtype=torch.int32, device=DEV), 1, 1, 1, 96, 0, 0.1, chunk=4)
+
+
+@pytest.mark.parametrize("sigmoid", [False, True])
+def test_more_single_tokens_than_arrival_counters(sigmoid):
+    """512 requests of 16 key heads are 8,192 pairs, twice the counters: chunks and sigmoid weights take the general kernel then."""
+    import types
+
+    from llm_b200.csrc import ops
+    B, G, D, page, chunk = 512, 16, 64, 16, 24
+    g = torch.Generator(device=DEV).manual_seed(2)
+    rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    lens = torch.randint(1, 3 * page, (B,), device=DEV, dtype=torch.int32, generator=g)
+    table = torch.arange(3 * B, dtype=torch.int32, device=DEV).view(B, 3)
+    kp, vp, q = rand(3 * B, G, page, D).bfloat16(), rand(3 * B, G, page, D).bfloat16(), rand(B, G * D).bfloat16()
+    kw = dict(chunk=chunk, sigmoid_bias=rand(G) - 1 if sigmoid else None)
+    ctx = types.SimpleNamespace(decode_only=True, kv_bucket=3 * page, n_entries=B, n_tokens=B, kv_lens=lens, positions=lens - 1,
+                                token_entry=torch.arange(B, dtype=torch.int32, device=DEV))
+    out = torch.full((B, G * D), float("nan"), device=DEV, dtype=torch.bfloat16)
+    ops.paged_attention(out, q, kp, vp, types.SimpleNamespace(block_table=table), ctx, G, G, D, 0, 0.125, **kw)
+    ref = torch.zeros(B, G * D, device=DEV)
+    ops.paged_attention_generic(ref, q.float(), kp.float(), vp.float(), table, ctx.token_entry, ctx.positions, B, G, G, D, 0, 0.125, **kw)
+    # float32 sums of at most 24 terms of size one, then the output's rounding
+    assert ((out.float() - ref).abs() <= ref.abs() * 2 ** -8 + 2e-5).all()
