@@ -14,6 +14,7 @@
 
 #include "common.cuh"
 #include "tcgen05.cuh"
+#include "warp_mma.cuh"
 
 namespace decode_mma {
 
@@ -57,23 +58,16 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// tanh, ln(1 + x) and the sigmoid without branches, for scores: a warp has a scheduler to itself here and walks a tile's 16 scores a lane
-// one after the other, so the library's functions (a branch each) cost more than the rest of the kernel: five requests of 1,100 keys
-// with cap and distance bias 32 us a launch with them, 24 us with these.  Absolute errors, from float32's own rounding: tanh 1.2e-7
-// (of a score that the cap then multiplies), ln 2e-7; the scores they enter carry the rounding of bfloat16 queries and keys.
-__device__ __forceinline__ float rcp(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
+// The sigmoid in float32 without the branch of the library's division, which keeps a tile's 16 scores a lane from running side by side:
+// 1 + e^-x by a step of Newton's iteration for the reciprocal on the hardware's approximation (which stands where the step would
+// overflow).  Every float32 number against 64 bits: the same largest error as 1 / (1 + expf(-x)) in every range down to -87 (3.43 units in the last
+// place of the smallest, 8.9e-8 absolute); below that the result is less than 1.2e-38 and may be 0.
+__device__ __forceinline__ float sigmoid_flat(float x) {
+  const float y = 1.f + expf(-x);
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
+  return y < 1e37f ? fmaf(r, fmaf(-y, r, 1.f), r) : r;
 }
-__device__ __forceinline__ float tanh_flat(float x) { return 1.f - 2.f * rcp(ex2(x * 2.885390081777927f) + 1.f); }      // 2 log2(e); +-1 at the ends
-__device__ __forceinline__ float log1p_flat(float x) {
-  float y;
-  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(1.f + x));
-  return y * 0.6931471805599453f;
-}
-__device__ __forceinline__ float sigmoid_flat(float x) { return rcp(1.f + ex2(x * -1.4426950408889634f)); }
-__device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<const uint32_t*>(&h);
@@ -99,7 +93,7 @@ __device__ __forceinline__ float2 sum2(const MaybePartial<__nv_bfloat16>& s, siz
 }
 
 // Scratch layout as in attention_decode.cu: counters, then ml [entries, heads, splits, 2] (the
-// maximum here in the base-2 domain of the pre-scaled scores), then o [entries, heads, splits, HS].
+// maximum here in the base-2 domain of the pre-scaled scores, with EXT of the scores), then o [entries, heads, splits, HS].
 //
 // CLUSTER: the CTAs of the ranges of one (request, kv head) form a thread-block cluster (2 to 8
 // along blockIdx.x).  They exchange their results through distributed shared memory (into the receivers' dynamic
@@ -125,13 +119,13 @@ struct FusedQkv {
 };
 
 // EXT: the options of the CUDA-core kernel (attention_decode.cu) and the sigmoid weights of the general one.  The visible keys
-// are walked as a list: the kept first keys, then the window's (or the chunk's); index u of the list is key u or u + skip.  P
-// stays what it was there, float32: it enters the second product as two bfloat16 numbers whose sum it is to 2^-18 (an output is
-// rounded to 2^-9; against 64 bits the error of both kernels is the same three digits, and the second MMA costs nothing that
-// shows: the kernel is bound by latency).  What a decode step gains, us a step, with the CUDA-core kernel (four or six launches of
-// 37 to 48 us) or the general one (two of 214 us, a warp per head) -> with this one: window, cap and sink, 3 requests of 1,900 keys,
-// 913 -> 824; distance bias and shared values, 5 requests of 1,100, 1,070 -> 932; latents with a learned sink and chunks of 256 with
-// sigmoid weights, 8 requests of 700, 1,402 -> 831.
+// are walked as a list: the kept first keys, then the window's (or the chunk's); index u of the list is key u or u + skip.  Scores and
+// weights are float32 numbers from the library's functions, as in those kernels, and P enters the second product as three bfloat16
+// numbers whose sum it is.  Against 64 bits the outputs that are not the correctly rounded ones are as many as theirs (0.02 to 0.03 %; with
+// two bfloat16 numbers and functions of hardware approximations 0.1 to 0.2 %, 1.4 % under a cap of 500).  Microseconds a launch, the CUDA-core
+// kernel or (sigmoid weights) two bfloat16 numbers and approximations -> this one: window, cap and sink, 3 requests of 1,900 keys, 43.9 -> 10.9;
+// cap, distance bias and shared values, 5 requests of 1,100, 52.7 -> 14.2; latents with a learned sink, 8 requests of 700, 68.1 -> 7.9;
+// chunks of 256 with sigmoid weights, head size 64, 4.15 -> 4.8 (a decode step with two of the general kernel's launches 1,402 us, with these 831).
 struct Options {
   float softcap;                 // > 0: scores pass cap * tanh(score / cap)
   int sink;                      // one more term in the denominator, of score sink_values[head] or 0
@@ -204,7 +198,8 @@ decode_attention_mma_kernel(__nv_bfloat16* __restrict__ out, long long out_strid
                             int n_entries, int n_heads, int n_kv, int page_size, int window, float scale_log2e, int splits,
                             FusedQkv fused, int kv_share, Options opt, int balance) {
   static_assert(!(FUSED && EXT), "the fused kernel has no options");
-  constexpr float LOG2E = 1.4426950408889634f;
+  // weights from scores: base 2 of scores that carry the factor already, or (EXT) the float32 exponential of the scores as they are
+  auto weight = [](float x) { return EXT ? expf(x) : ex2(x); };
   constexpr int KS = HS / 16;                  // k-steps of Q K^T
   constexpr int DT = HS / 8;                   // 8-wide tiles of the output row
   constexpr int CH = HS / 8;                   // 16-byte chunks of a row
@@ -393,8 +388,8 @@ decode_attention_mma_kernel(__nv_bfloat16* __restrict__ out, long long out_strid
   auto finish = [&](int head, float m, float l, float acc) -> float {
     if (EXT && opt.sigmoid_bias) return acc;
     if (EXT && opt.sink) {
-      const float sv = (opt.sink_values ? opt.sink_values[head] : 0.f) * LOG2E, top = fmaxf(m, sv), f = ex2(m - top);
-      return acc * f / (l * f + ex2(sv - top));
+      const float sv = opt.sink_values ? opt.sink_values[head] : 0.f, top = fmaxf(m, sv), f = weight(m - top);
+      return acc * f / (l * f + weight(sv - top));
     }
     return acc / l;
   };
@@ -531,43 +526,36 @@ decode_attention_mma_kernel(__nv_bfloat16* __restrict__ out, long long out_strid
       }
       // ---- scale, mask the keys past the range, running maximum and sum ----
       float t0 = -INFINITY, t1 = -INFINITY;
+      // EXT: what the options make of the scores.  Rolled over the tile's four parts, a part of which goes to the end of the array when it is made:
+      // inside a decode step the code is fetched once a launch (3 requests of 1,900 keys, cap and sink: a step of four launches 725 us unrolled,
+      // 715 rolled; 8 requests with sigmoid weights 620 and 615)
       if constexpr (EXT) {                                         // scale_log2e is the plain scale here
+#pragma unroll 1
+        for (int nt = 0; nt < 4; ++nt) {
+          float x[4];
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) s[nt][i] *= scale_log2e;
-        if (opt.softcap > 0.f) {
-#pragma unroll
-          for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) s[nt][i] = opt.softcap * tanh_flat(s[nt][i] * inv_cap);
-        }
-        if (dist) {
-#pragma unroll
-          for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-              const float away = (float)(pos - position_of(t + nt * 8 + qcol + j));
-              s[nt][j] -= ra0 * log1p_flat(rb0 * away);
-              s[nt][2 + j] -= ra1 * log1p_flat(rb1 * away);
+          for (int i = 0; i < 4; ++i) {
+            x[i] = s[0][i] * scale_log2e;
+            if (opt.softcap > 0.f) x[i] = opt.softcap * tanhf(x[i] * inv_cap);
+            if (dist) {
+              const float away = (float)(pos - position_of(t + nt * 8 + qcol + (i & 1)));
+              x[i] -= (i < 2 ? ra0 : ra1) * log1pf((i < 2 ? rb0 : rb1) * away);
             }
-        }
-        if (gated) {                                               // the weights themselves; nothing is exponentiated below
+            if (gated) x[i] = sigmoid_flat(x[i] + (i < 2 ? ra0 : ra1));
+          }
 #pragma unroll
-          for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) s[nt][i] = sigmoid_flat(s[nt][i] + (i < 2 ? ra0 : ra1));
+          for (int i = 0; i < 4; ++i) { s[0][i] = s[1][i]; s[1][i] = s[2][i]; s[2][i] = s[3][i]; s[3][i] = x[i]; }
         }
       }
-      const float to_base2 = EXT ? (gated ? 1.f : LOG2E) : scale_log2e, none = gated ? 0.f : -INFINITY;
+      const float factor = EXT ? 1.f : scale_log2e, none = gated ? 0.f : -INFINITY;
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt) {
         const int kp = t + nt * 8 + qcol;
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const bool valid = kp + j < k_end;
-          s[nt][j] = valid ? s[nt][j] * to_base2 : none;
-          s[nt][2 + j] = valid ? s[nt][2 + j] * to_base2 : none;
+          s[nt][j] = valid ? s[nt][j] * factor : none;
+          s[nt][2 + j] = valid ? s[nt][2 + j] * factor : none;
           t0 = fmaxf(t0, s[nt][j]);
           t1 = fmaxf(t1, s[nt][2 + j]);
         }
@@ -578,42 +566,57 @@ decode_attention_mma_kernel(__nv_bfloat16* __restrict__ out, long long out_strid
       t1 = fmaxf(t1, __shfl_xor_sync(0xffffffffu, t1, 2));
       // finite: the tile holds at least one key.  Sigmoid weights have no maximum: 0, and factors of 1
       const float n0 = gated ? 0.f : fmaxf(m0, t0), n1 = gated ? 0.f : fmaxf(m1, t1);
-      const float a0 = gated ? 1.f : ex2(m0 - n0), a1 = gated ? 1.f : ex2(m1 - n1);
+      const float a0 = gated ? 1.f : weight(m0 - n0), a1 = gated ? 1.f : weight(m1 - n1);
       m0 = n0; m1 = n1;
       l0 *= a0; l1 *= a1;
 #pragma unroll
       for (int d = 0; d < DT; ++d) { o[d][0] *= a0; o[d][1] *= a0; o[d][2] *= a1; o[d][3] *= a1; }
-      uint32_t pf[2][4];                                          // P as the A operand of two k-steps of 16 keys
-      uint32_t pl[2][EXT ? 4 : 1];                                // EXT: what its rounding left, rounded in turn
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt) {
-        const float p0 = gated ? s[nt][0] : ex2(s[nt][0] - n0), p1 = gated ? s[nt][1] : ex2(s[nt][1] - n0);
-        const float p2 = gated ? s[nt][2] : ex2(s[nt][2] - n1), p3 = gated ? s[nt][3] : ex2(s[nt][3] - n1);
-        if constexpr (EXT) {
-          pl[nt >> 1][(nt & 1) * 2] = pack2(p0 - round_bf16(p0), p1 - round_bf16(p1));
-          pl[nt >> 1][(nt & 1) * 2 + 1] = pack2(p2 - round_bf16(p2), p3 - round_bf16(p3));
+        if (!gated) {
+          s[nt][0] = weight(s[nt][0] - n0); s[nt][1] = weight(s[nt][1] - n0);
+          s[nt][2] = weight(s[nt][2] - n1); s[nt][3] = weight(s[nt][3] - n1);
         }
-        l0 += p0 + p1;
-        l1 += p2 + p3;
-        pf[nt >> 1][(nt & 1) * 2] = pack2(p0, p1);
-        pf[nt >> 1][(nt & 1) * 2 + 1] = pack2(p2, p3);
+        l0 += s[nt][0] + s[nt][1];
+        l1 += s[nt][2] + s[nt][3];
       }
       // ---- O += P V ----
+      // EXT: P as three bfloat16 numbers, whose sum it is, and GV 16-column parts of the output at a time, so that the three products of an
+      // accumulator, each waiting for the one before, run among those of others (5 requests of 1,100 keys: unrolled, one part at a time 14.2 us, this way 13.7)
+      constexpr int PN = EXT ? 3 : 1, GV = EXT ? 4 : 1;
       const int mid = lane >> 3, r8 = lane & 7;
 #pragma unroll
       for (int kk = 0; kk < 2; ++kk) {
+        uint32_t pf[PN][4];                                        // P as the A operand of a k-step of 16 keys
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const float x = s[kk * 2 + (r >> 1)][(r & 1) * 2], y = s[kk * 2 + (r >> 1)][(r & 1) * 2 + 1];
+          if constexpr (EXT) {
+            uint32_t parts[3];
+            split3(x, y, parts);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) pf[i][r] = parts[i];
+          } else {
+            pf[0][r] = pack2(x, y);
+          }
+        }
         const int kl = kk * 16 + (mid & 1) * 8 + r8;               // the key whose row this lane points at
 #pragma unroll
-        for (int dp = 0; dp < DT / 2; ++dp) {
-          const int c = dp * 2 + (mid >> 1);
-          const int cs = (c & ~7) | ((c ^ kl) & 7);
-          uint32_t vb[4];
-          ldmatrix_x4_trans(vb, v_addr + kl * (HS * 2) + cs * 16);
-          mma_16816(o[dp * 2], pf[kk], vb[0], vb[1]);
-          mma_16816(o[dp * 2 + 1], pf[kk], vb[2], vb[3]);
-          if constexpr (EXT) {
-            mma_16816(o[dp * 2], pl[kk], vb[0], vb[1]);
-            mma_16816(o[dp * 2 + 1], pl[kk], vb[2], vb[3]);
+        for (int dp = 0; dp < DT / 2; dp += GV) {
+          uint32_t vb[GV][4];
+#pragma unroll
+          for (int u = 0; u < GV; ++u) {
+            const int c = (dp + u) * 2 + (mid >> 1);
+            const int cs = (c & ~7) | ((c ^ kl) & 7);
+            ldmatrix_x4_trans(vb[u], v_addr + kl * (HS * 2) + cs * 16);
+          }
+#pragma unroll
+          for (int i = PN - 1; i >= 0; --i) {                      // the small parts first
+#pragma unroll
+            for (int u = 0; u < GV; ++u) {
+              mma_16816(o[(dp + u) * 2], pf[i], vb[u][0], vb[u][1]);
+              mma_16816(o[(dp + u) * 2 + 1], pf[i], vb[u][2], vb[u][3]);
+            }
           }
         }
       }
@@ -644,7 +647,7 @@ decode_attention_mma_kernel(__nv_bfloat16* __restrict__ out, long long out_strid
       for (int w = 0; w < 4; ++w) m = fmaxf(m, wm_s[w][tid]);
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
-        const float f = wm_s[w][tid] > -INFINITY ? ex2(wm_s[w][tid] - m) : 0.f;
+        const float f = wm_s[w][tid] > -INFINITY ? weight(wm_s[w][tid] - m) : 0.f;
         l += f * wl_s[w][tid];
         wm_s[w][tid] = f;
       }
@@ -698,7 +701,7 @@ decode_attention_mma_kernel(__nv_bfloat16* __restrict__ out, long long out_strid
         for (int r = 0; r < splits; ++r) {                          // in the order of the ranges
           const float mr = w_s[h][r];
           if (mr > -INFINITY) {
-            const float f = ex2(mr - m);
+            const float f = weight(mr - m);
             l += f * l_in[h][r];
             acc += f * recv_s[r * part + j];
           }
@@ -732,12 +735,12 @@ decode_attention_mma_kernel(__nv_bfloat16* __restrict__ out, long long out_strid
     }
     __syncthreads();
     if (tid < nh) {
-      const float sv = !EXT || !opt.sink ? -INFINITY : (opt.sink_values ? opt.sink_values[g * group + h0 + tid] : 0.f) * LOG2E;
+      const float sv = !EXT || !opt.sink ? -INFINITY : (opt.sink_values ? opt.sink_values[g * group + h0 + tid] : 0.f);
       float m = sv;                                               // the sink is one more range: maximum its score, sum 1, no values
       for (int sp = 0; sp < n_active; ++sp) m = fmaxf(m, w_s[tid][sp]);
-      float l = EXT && opt.sink ? ex2(sv - m) : 0.f;
+      float l = EXT && opt.sink ? weight(sv - m) : 0.f;
       for (int sp = 0; sp < n_active; ++sp) {
-        const float f = ex2(w_s[tid][sp] - m);
+        const float f = weight(w_s[tid][sp] - m);
         l += f * l_in[tid][sp];
         w_s[tid][sp] = f;
       }

@@ -97,3 +97,54 @@ def test_more_single_tokens_than_arrival_counters(sigmoid):
     ops.paged_attention_generic(ref, q.float(), kp.float(), vp.float(), table, ctx.token_entry, ctx.positions, B, G, G, D, 0, 0.125, **kw)
     # float32 sums of at most 24 terms of size one, then the output's rounding
     assert ((out.float() - ref).abs() <= ref.abs() * 2 ** -8 + 2e-5).all()
+
+
+def exact(q, kp, vp, table, lens, H, G, D, window, scale, o):
+    """The attention of single tokens in 64 bits."""
+    ref = torch.zeros(len(lens), H, D, dtype=torch.float64, device=DEV)
+    column = lambda t: t.double()[:, None]
+    for b, n in enumerate(lens):
+        at = table[b].long()
+        K, V = ([t[at].permute(1, 0, 2, 3).flatten(1, 2)[:, :n].double().repeat_interleave(H // t.shape[1], 0) for t in (kp, vp)])
+        s, away = (q[b].view(H, 1, D).double() * K).sum(-1) * scale, n - 1 - torch.arange(n, device=DEV)
+        seen = (away < window) | (torch.arange(n, device=DEV) < o["keep_first"]) if window else away >= 0
+        if o["chunk"]:
+            seen = torch.arange(n, device=DEV) // o["chunk"] == (n - 1) // o["chunk"]
+        if o["softcap"]:
+            s = o["softcap"] * torch.tanh(s / o["softcap"])
+        if o["dist_bias"]:
+            s = s - column(o["dist_bias"][0]) * torch.log1p(column(o["dist_bias"][1]) * away.double())
+        if o["sigmoid_bias"] is not None:
+            p = torch.sigmoid(s + column(o["sigmoid_bias"])) * seen
+        else:
+            sink = s[:, :0] if not o["sink"] else torch.zeros_like(s[:, :1]) if o["sink_values"] is None else column(o["sink_values"])
+            p = torch.softmax(torch.cat([s.masked_fill(~seen, -math.inf), sink], 1), -1)[:, :n]
+        ref[b] = torch.einsum("hk,hkd->hd", p, V)
+    return ref.flatten(1)
+
+
+@pytest.mark.parametrize("case", [(16, 4, 128, dict(window=1024, softcap=40.0, sink=True, keep_first=8)), (16, 4, 128, dict(softcap=8.0)),
+                                  (16, 4, 128, dict(softcap=500.0)), (20, 4, 128, dict(softcap=30.0, dist=True, v_share=2)), (16, 4, 64, dict(dist=True)),
+                                  (16, 4, 64, dict(chunk=256, sigmoid=True)), (16, 4, 128, dict(sigmoid=True)), (16, 1, 128, dict(window=1024, sink="learned"))])
+def test_scores_and_weights_keep_the_precision_of_float32(case):
+    """How many outputs are not the exact value rounded once to bfloat16: no more than twice as many (and a dozen) as those of the general
+    kernel, whose scores, weights and sums are float32 numbers.  Weights of sixteen bits, or functions with an absolute error under a large cap,
+    give several times as many (five to fifty)."""
+    from llm_b200.csrc import ops
+    H, G, D, o = case
+    g = torch.Generator(device=DEV).manual_seed(H + D)
+    rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    lens, page, share, w = [1900, 1500, 1024, 700, 1, 33] * 4, 16, o.get("v_share", 1), o.get("window", 0)
+    B, width = len(lens), -(-max(lens) // page)
+    kp, vp = rand(B * width, G, page, D).bfloat16(), rand(B * width, G // share, page, D).bfloat16()
+    table = torch.randperm(B * width, device=DEV, generator=g).to(torch.int32).view(B, width)
+    q, kv_lens = (rand(B, H * D) * 1.5).bfloat16(), torch.tensor(lens, dtype=torch.int32, device=DEV)
+    kw = dict(softcap=o.get("softcap", 0.0), sink=bool(o.get("sink")), keep_first=o.get("keep_first", 0), v_share=share, chunk=o.get("chunk", 0),
+              sink_values=rand(H) * 2 if o.get("sink") == "learned" else None, sigmoid_bias=rand(H) - 3 if o.get("sigmoid") else None,
+              dist_bias=(rand(H).abs(), rand(H).abs()) if o.get("dist") else None)
+    best = exact(q, kp, vp, table, lens, H, G, D, w, D ** -0.5, kw).bfloat16()
+    out, general = torch.zeros_like(q), torch.zeros_like(q)
+    ops.paged_attention_decode(out, q, kp, vp, table, kv_lens, B, H, G, D, w, D ** -0.5, splits=6, **kw)
+    ops.paged_attention_generic(general, q, kp, vp, table, torch.arange(B, dtype=torch.int32, device=DEV), kv_lens - 1, B, H, G, D, w, D ** -0.5, **kw)
+    off = lambda t: int((t != best).sum())
+    assert off(out) <= 2 * off(general) + 12, (off(out), off(general), best.numel())
