@@ -12,8 +12,12 @@
 // multiply-adds, a running product per (s, d).  The three contractions run as bfloat16 MMAs on operands split into three
 // bfloat16 numbers each (v is bfloat16 to begin with): S^T q takes the six products above 2^-24, the others three, summed in
 // float32; S itself stays in float32 registers as MMA accumulators of S^T, which are in the layout of the next product's operand,
-// and the decay and sum of the update are float32 multiply-adds.  A token that is not finite reaches the tokens of its own chunk
-// and the later ones of its request.
+// and the decay and sum of the update are float32 multiply-adds.
+//
+// What is not finite reaches its own token and the later ones of its request, as token by token: queries, keys and decays do by the
+// form of the sums (a weight of a later token is set to 0, not multiplied), but a value that is infinite or no number would meet the
+// zeros of the earlier tokens' rows of A in the MMA.  From a chunk on that holds one in the CTA's columns, the segment is walked token by
+// token (walk_rest), which a healthy model never sees; looking for one costs nothing that shows (a piece of 16 bytes a thread and chunk).
 //
 // Work split: a CTA owns (segment of an entry, head, 16 value columns a warp).  Segments run side by side in two passes as in
 // scan.cu: pass 1 leaves the end state from zero and the product of the decays of every segment but an entry's last, a chain
@@ -40,6 +44,13 @@ constexpr int MAX_SEG = 256;             // tokens of a segment (the scalar form
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 __device__ __forceinline__ float log_sigmoid_f(float z) { return fminf(z, 0.f) - log1pf(expf(-fabsf(z))); }
 
+// Whether one of eight bfloat16 numbers is infinite or no number.
+__device__ __forceinline__ bool not_finite8(const bf16* p) {
+  const uint4 w = *reinterpret_cast<const uint4*>(p);
+  auto two = [](uint32_t x) { return (x & 0x7f80u) == 0x7f80u || (x & 0x7f800000u) == 0x7f800000u; };
+  return two(w.x) || two(w.y) || two(w.z) || two(w.w);
+}
+
 // Segment `index` of the step: its entry and tokens [t0, t1).  False behind the last one.
 __device__ __forceinline__ bool segment_of(const int* cu, int n_entries, int seg_len, int index, int& entry, int& t0, int& t1, int& end) {
   int b = cu[0];
@@ -57,6 +68,63 @@ __device__ __forceinline__ bool segment_of(const int* cu, int n_entries, int seg
   return false;
 }
 
+// The tokens [from, t1) of a segment one after the other, a thread per value column: the state starts and stays in the segment's place,
+// from where it goes to the request's if the segment is its entry's last.  rows: shared memory for 3 * dim numbers; decays: thread d's
+// product of pass 1 so far.
+template <int FORM, bool STATE_ONLY>
+__device__ void walk_rest(const Args& a, float* rows, int entry, int from, int t1, bool last, int colb, int vt, float decays) {
+  const int tid = threadIdx.x, head = blockIdx.y, qk_head = head / (a.heads / a.qk_heads), dim = a.dim, vdim = a.vdim;
+  const size_t unit = (size_t)blockIdx.z * a.heads + head;
+  float *a_s = rows, *q_s = rows + dim, *k_s = rows + 2 * dim;
+  const int col = colb + tid;
+  const bool live = tid < vt && col < vdim;
+  float* S = a.seg_state + unit * dim * vdim + col;
+  for (int t = from; t < t1; ++t) {
+    __syncthreads();
+    for (int d = tid; d < dim; d += blockDim.x) {
+      const size_t at = (size_t)t * a.qk_stride + (size_t)qk_head * dim + d;
+      float av, qv = __bfloat162float(a.q[at]), kv = FORM == GATE ? 0.f : __bfloat162float(a.k[at]);
+      if (FORM == SCALAR) {
+        const float dt = softplus_f(__bfloat162float(a.dt[(size_t)t * a.dt_stride + head]) + a.dt_bias[head]);
+        av = expf(-expf(a.a_log[head]) * dt);
+        kv *= dt;
+      } else {
+        const float z = a.z[(size_t)t * a.z_stride + (size_t)head * dim + d] + (a.z_bias ? a.z_bias[head * dim + d] : 0.f);
+        if (FORM == BONUS) {
+          av = expf(-expf(z));
+        } else if (FORM == POWER) {
+          av = expf(log_sigmoid_f(z) * a.inv_tau);
+        } else {
+          const float low = a.bonus[head * dim + d];
+          qv = qv / (1.f + expf(-qv));
+          av = low + (1.f - low) / (1.f + expf(-z));
+          kv = 1.f - av;
+        }
+      }
+      a_s[d] = av; q_s[d] = qv; k_s[d] = kv;
+      decays *= av;                                                    // dim <= blockDim.x: one channel a thread
+    }
+    __syncthreads();
+    if (!live) continue;
+    const float v = __bfloat162float(a.v[(size_t)t * a.v_stride + (size_t)head * vdim + col]);
+    float o = 0.f;
+    for (int d = 0; d < dim; ++d) {
+      const float old = S[(size_t)d * vdim], kv = k_s[d] * v, now = fmaf(a_s[d], old, kv);
+      o = fmaf(q_s[d], FORM == BONUS ? fmaf(a.bonus[head * dim + d], kv, old) : now, o);
+      S[(size_t)d * vdim] = now;
+    }
+    if (FORM == POWER) o *= a.q_scale;
+    if (FORM == SCALAR) o = fmaf(a.skip[head], v, o);
+    if (!STATE_ONLY) a.out[(size_t)t * a.out_stride + (size_t)head * vdim + col] = o;
+  }
+  if (STATE_ONLY) {
+    if (blockIdx.x == 0 && tid < dim) a.seg_decay[unit * dim + tid] = decays;
+  } else if (last && live) {
+    float* to = a.state + (size_t)a.state_slots[entry] * a.slot_stride + (size_t)head * dim * vdim + col;
+    for (int d = 0; d < dim; ++d) to[(size_t)d * vdim] = S[(size_t)d * vdim];
+  }
+}
+
 // ---- scalar form ----------------------------------------------------------------------------------------------
 // One decay per head and token: it comes out of every contraction.  q and k enter as they are (bfloat16), A = (q . k) times the product
 // of the decays between, which is one number per pair of tokens, and the update's scale stands on v:
@@ -71,7 +139,7 @@ struct ScalarShape {
 
 template <int DP, bool STATE_ONLY>
 __global__ void __launch_bounds__(128, 4)
-scalar_chunk_kernel(const Args a) {
+scalar_chunk_kernel(const __grid_constant__ Args a) {
   using Sh = ScalarShape<DP>;
   constexpr int NT = Sh::NT, VT = Sh::VT, VP = Sh::VP, SP = Sh::SP;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -145,13 +213,15 @@ scalar_chunk_kernel(const Args a) {
   float decays = 1.f;
   const int tr = (lane & 7) + ((lane >> 3) & 1) * 8, th = (lane >> 4) * 8;      // ldmatrix: rows by lane bit 3, halves by bit 4
   const int hr = (lane & 7) + (lane >> 4) * 8, hh = ((lane >> 3) & 1) * 8;      // the other way round
-  for (int ch = 0; ch < chunks; ++ch) {
+  static_assert(C * VT / 8 == NT, "a thread looks at what it brought itself: one piece of the values");
+  int ch = 0;
+  for (; ch < chunks; ++ch) {
     const int c0 = t0 + ch * C, n = min(C, t1 - c0);
-    cp_async_wait_all();
-    __syncthreads();
-    if (ch + 1 < chunks) bring(c0 + C, (ch + 1) & 1);
     const bf16* q_r = reinterpret_cast<const bf16*>(smem + (ch & 1) * Sh::STAGE);
     const bf16 *k_r = q_r + C * SP, *v_r = k_r + C * SP;
+    cp_async_wait_all();
+    if (__syncthreads_or(not_finite8(v_r + tid / (VT / 8) * VP + tid % (VT / 8) * 8))) break;
+    if (ch + 1 < chunks) bring(c0 + C, (ch + 1) & 1);
     const float *P = p_s + ch * C, *D = d_s + ch * C * C;
     uint32_t va[4];
     ldsm4_t(va, v_r + hr * VP + wcol + hh);
@@ -246,8 +316,9 @@ scalar_chunk_kernel(const Args a) {
         for (int e = 0; e < 4; ++e) st[2 * i + j][e] = fmaf(st[2 * i + j][e], pc, u[j][e]);
     }
   }
-  if (!STATE_ONLY && !last) return;
-  float* S_out = STATE_ONLY ? S_seg : a.state + (size_t)a.state_slots[entry] * a.slot_stride + (size_t)head * dim * vdim;
+  const bool rest = ch < chunks;                                       // a chunk that is not finite
+  if (!STATE_ONLY && !last && !rest) return;
+  float* S_out = STATE_ONLY || rest ? S_seg : a.state + (size_t)a.state_slots[entry] * a.slot_stride + (size_t)head * dim * vdim;
 #pragma unroll
   for (int i = 0; i < DP / 8; ++i) {
 #pragma unroll
@@ -255,6 +326,11 @@ scalar_chunk_kernel(const Args a) {
       const int dd = i * 8 + dc + (j & 1), vv = vr + (j >> 1) * 8;
       if (dd < dim && vv < vdim) S_out[(size_t)dd * vdim + vv] = st[i][j];
     }
+  }
+  if (rest) {
+    __syncthreads();
+    walk_rest<SCALAR, STATE_ONLY>(a, reinterpret_cast<float*>(smem), entry, t0 + ch * C, t1, last, colb, VT, decays);
+    return;
   }
   if (STATE_ONLY && blockIdx.x == 0) {
     for (int d = tid; d < dim; d += NT) a.seg_decay[unit * dim + d] = decays;
@@ -274,7 +350,7 @@ struct Shape {
 
 template <int FORM, int DP, int WARPS, bool STATE_ONLY>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : DP == 128 ? 2 : 4)
-diag_chunk_kernel(const Args a) {
+diag_chunk_kernel(const __grid_constant__ Args a) {
   using Sh = Shape<DP, WARPS>;
   constexpr int NT = Sh::NT, VT = Sh::VT, VP = Sh::VP, SP = Sh::SP;
   constexpr bool HAS_K = FORM != GATE;
@@ -348,15 +424,17 @@ diag_chunk_kernel(const Args a) {
     }
   }
   float decays = 1.f;                                                  // pass 1: the segment's product, channel d
-  int stage = 0;
-  for (int c0 = t0; c0 < t1; c0 += C, stage ^= 1) {
+  static_assert(C * VT / 8 == NT, "a thread looks at what it brought itself: one piece of the values");
+  int stage = 0, c0 = t0;
+  for (; c0 < t1; c0 += C, stage ^= 1) {
     const int n = min(C, t1 - c0);
-    cp_async_wait_all();
-    __syncthreads();                                                   // this chunk is here; the last one's operands are read
-    if (c0 + C < t1) bring(c0 + C, stage ^ 1);
     const unsigned char* base = smem + stage * Sh::STAGE;
     const float* z_r = reinterpret_cast<const float*>(base);
     const bf16 *q_r = reinterpret_cast<const bf16*>(base + Sh::Z), *k_r = q_r + C * DP, *v_r = k_r + C * DP;
+    cp_async_wait_all();
+    // behind the barrier this chunk is here and the last one's operands are read
+    if (__syncthreads_or(not_finite8(v_r + tid / (VT / 8) * VP + tid % (VT / 8) * 8))) break;
+    if (c0 + C < t1) bring(c0 + C, stage ^ 1);
     // decays, queries and keys in float32; tokens behind the end and channels behind dim: a = 1, q = k = 0
 #pragma unroll 4
     for (int c = tid / DP; c < C; c += NT / DP) {
@@ -559,8 +637,9 @@ diag_chunk_kernel(const Args a) {
       }
     }
   }
-  if (!STATE_ONLY && !last) return;
-  float* S_out = STATE_ONLY ? S_seg : a.state + (size_t)a.state_slots[entry] * a.slot_stride + (size_t)head * dim * vdim;
+  const bool rest = c0 < t1;                                           // a chunk that is not finite
+  if (!STATE_ONLY && !last && !rest) return;
+  float* S_out = STATE_ONLY || rest ? S_seg : a.state + (size_t)a.state_slots[entry] * a.slot_stride + (size_t)head * dim * vdim;
 #pragma unroll
   for (int i = 0; i < DP / 8; ++i) {
 #pragma unroll
@@ -568,6 +647,11 @@ diag_chunk_kernel(const Args a) {
       const int dd = i * 8 + dc + (j & 1), vv = vr + (j >> 1) * 8;
       if (dd < dim && vv < vdim) S_out[(size_t)dd * vdim + vv] = st[i][j];
     }
+  }
+  if (rest) {
+    __syncthreads();
+    walk_rest<FORM, STATE_ONLY>(a, a_s, entry, c0, t1, last, colb, VT, decays);
+    return;
   }
   if (STATE_ONLY && blockIdx.x == 0 && tid < dim) a.seg_decay[unit * dim + d] = decays;
 }
