@@ -26,10 +26,10 @@
 // What bounds it: latency at 16 (eight-warp form) or 8 to 16 warps an SM: half of the issue slots and a fifth of the tensor pipe are in use
 // (what the warps wait for is shared memory and the barriers between a chunk's three parts).  2,048 tokens, the three launches against
 // the token-by-token passes that they took the place of: power form, 8 heads of 128 x 256: 261 -> 132 us; bonus form, 32 heads of
-// 64 x 64: 214 -> 94; scalar form, 32 heads of 128 x 64: 245 -> 74; gate form, 16 heads of 128 x 128: 350 -> 123.  Seven entries of 1
+// 64 x 64: 214 -> 103; scalar form, 32 heads of 128 x 64: 245 -> 74; gate form, 16 heads of 128 x 128: 350 -> 123.  Seven entries of 1
 // to 150 tokens, 8 heads of 32 x 32: 54 -> 39; heads of 8 x 8: 149 -> 39 (the tiles are then mostly padding, and still ahead).
-// Errors against 64 bits (relative, outputs / states): power form 7.8e-7 / 8.8e-7 -> 7.1e-7 / 8.4e-7, bonus form 1.1e-7 / 8.4e-8 ->
-// 1.05e-7 / 8.7e-8, scalar form 1.7e-7 / 1.4e-7 -> 1.7e-7 / 1.3e-7, gate form 1.7e-7 / 3.6e-7 -> 1.6e-7 / 2.8e-7.
+// Errors against 64 bits (relative, outputs / states): power form 7.8e-7 / 8.7e-7 -> 7.1e-7 / 8.4e-7, bonus form 1.1e-7 / 8.4e-8 ->
+// 1.0e-7 / 6.8e-8, scalar form 1.7e-7 / 1.4e-7 -> 1.7e-7 / 1.3e-7, gate form 1.7e-7 / 3.2e-7 -> 1.6e-7 / 2.8e-7.
 #include "diag_chunk.cuh"
 #include "warp_mma.cuh"
 
@@ -363,6 +363,7 @@ diag_chunk_kernel(const __grid_constant__ Args a) {
   bf16* A_s = kr_s + 3 * C * SP;                                       // [3][C][AP]
   float* p_s = reinterpret_cast<float*>(A_s + 3 * C * AP);             // [DP]
   float* u_s = p_s + DP;                                               // bonus form: u [DP]
+  float* e_s = u_s + DP;                                               // and the exponents of the decays, a = exp(-e) [C][DP]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int head = blockIdx.y, qk_head = head / (a.heads / a.qk_heads);
   const int dim = a.dim, vdim = a.vdim, colb = blockIdx.x * VT;
@@ -423,7 +424,7 @@ diag_chunk_kernel(const __grid_constant__ Args a) {
       st[i][j] = (!STATE_ONLY && dd < dim && vv < vdim) ? S_seg[(size_t)dd * vdim + vv] : 0.f;
     }
   }
-  float decays = 1.f;                                                  // pass 1: the segment's product, channel d
+  float decays = FORM == BONUS ? 0.f : 1.f;                            // pass 1: the segment's product (bonus: exponent), channel d
   static_assert(C * VT / 8 == NT, "a thread looks at what it brought itself: one piece of the values");
   int stage = 0, c0 = t0;
   for (; c0 < t1; c0 += C, stage ^= 1) {
@@ -438,12 +439,13 @@ diag_chunk_kernel(const __grid_constant__ Args a) {
     // decays, queries and keys in float32; tokens behind the end and channels behind dim: a = 1, q = k = 0
 #pragma unroll 4
     for (int c = tid / DP; c < C; c += NT / DP) {
-      float av = 1.f, qv = 0.f, kv = 0.f;
+      float av = 1.f, qv = 0.f, kv = 0.f, ev = 0.f;
       if (c < n && d < dim) {
         if (!STATE_ONLY) qv = __bfloat162float(q_r[c * DP + d]);
         if (HAS_K) kv = __bfloat162float(k_r[c * DP + d]);
         if (FORM == BONUS) {
-          av = expf(-expf(z_r[c * DP + d] + zb));
+          ev = expf(z_r[c * DP + d] + zb);
+          av = expf(-ev);
         } else if (FORM == POWER) {
           av = expf(log_sigmoid_f(z_r[c * DP + d] + zb) * a.inv_tau);
         } else {
@@ -453,6 +455,7 @@ diag_chunk_kernel(const __grid_constant__ Args a) {
         }
       }
       a_s[c * DP + d] = av;
+      if (FORM == BONUS) e_s[c * DP + d] = ev;
       if (!STATE_ONLY) q_s[c * DP + d] = qv;
       k_s[c * DP + d] = kv;
     }
@@ -520,10 +523,17 @@ diag_chunk_kernel(const __grid_constant__ Args a) {
     }
     // q P (forward) and k R (backward), split.  A product is kept from what it lacks to one while that is less than a half: with
     // decays close to one the plain product's roundings were most of the state's error (gate form, 2,048 tokens, against 64 bits:
-    // plain 5.2e-7, token by token 3.2e-7, this way 2.8e-7).
+    // plain 5.2e-7, token by token 3.2e-7, this way 2.8e-7).  The bonus form has the decays' exponents at hand and sums those: a product
+    // is rounded once then, however many tokens it spans (32 heads of 64 x 64: token by token 8.4e-8, products 8.7e-8, this way 6.8e-8; 93
+    // us for the three launches with products, 103 this way).
     for (int task = tid; task < (STATE_ONLY ? DP : 2 * DP); task += NT) {
       float f = 1.f, lack = 0.f;
       auto on = [&](int t) {                                           // f <- f a_t
+        if (FORM == BONUS) {
+          lack += e_s[t * DP + d];
+          f = expf(-lack);
+          return;
+        }
         const float av = a_s[t * DP + d];
         lack = fmaf(1.f - av, f, lack);
         f = lack < 0.5f ? 1.f - lack : f * av;
@@ -564,7 +574,7 @@ diag_chunk_kernel(const __grid_constant__ Args a) {
           }
         }
         p_s[d] = f;
-        if (STATE_ONLY) decays *= f;
+        if (STATE_ONLY) decays = FORM == BONUS ? decays + lack : decays * f;
       }
     }
     __syncthreads();
@@ -637,6 +647,7 @@ diag_chunk_kernel(const __grid_constant__ Args a) {
       }
     }
   }
+  if (FORM == BONUS) decays = expf(-decays);
   const bool rest = c0 < t1;                                           // a chunk that is not finite
   if (!STATE_ONLY && !last && !rest) return;
   float* S_out = STATE_ONLY || rest ? S_seg : a.state + (size_t)a.state_slots[entry] * a.slot_stride + (size_t)head * dim * vdim;
@@ -713,7 +724,8 @@ int launch_passes(Kernel ends, Kernel outs, const Args& a, int vt, int threads, 
 template <int FORM, int DP, int WARPS>
 int launch_shape(const Args& a, int segs, cudaStream_t stream) {
   using Sh = Shape<DP, WARPS>;
-  return launch_passes(diag_chunk_kernel<FORM, DP, WARPS, true>, diag_chunk_kernel<FORM, DP, WARPS, false>, a, Sh::VT, Sh::NT, Sh::BYTES, segs, stream);
+  return launch_passes(diag_chunk_kernel<FORM, DP, WARPS, true>, diag_chunk_kernel<FORM, DP, WARPS, false>, a, Sh::VT, Sh::NT,
+                       Sh::BYTES + (FORM == BONUS ? Sh::F32 : 0), segs, stream);
 }
 
 template <int DP>
