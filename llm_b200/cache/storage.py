@@ -92,7 +92,7 @@ class StateStorage:
             return
         if self._regions.is_cuda:
             from ..csrc import ops
-            ops.zero_slots(self._regions, self._most_bytes, slots)
+            ops.zero_slots(self._regions, self._most_bytes, slots, self.tensors[0].shape[0])
         else:
             for t in self.tensors:
                 t[slots] = 0

@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import operator
 import os
 from ctypes import c_float, c_int, c_longlong, c_void_p
 
@@ -151,8 +152,14 @@ def embedding(resid: torch.Tensor, table: torch.Tensor, ids: torch.Tensor, n_tok
                                         c_int(vocab), c_int(_kind(table.dtype)), _ptr(status), c_float(scale), _stream()))
 
 
-def zero_slots(regions: torch.Tensor, most_bytes: int, slots) -> None:
-    """Zero the given slots of every tensor of `regions` (int64 [tensors, 2] on the device: address of slot 0, bytes of a slot)."""
+def zero_slots(regions: torch.Tensor, most_bytes: int, slots, held: int) -> None:
+    """Zero the given slots of every tensor of `regions` (int64 [tensors, 2] on the device: address of slot 0, bytes of a slot), each of
+    which has `held` slots.  Slots are numbered as Python indexes them: from -held to held - 1."""
+    slots = [operator.index(s) for s in slots]
+    for s in slots:
+        if not -held <= s < held:
+            raise IndexError(f"slot {s} of {held}")
+    slots = [s % held for s in slots]
     assert regions.dtype == torch.int64 and regions.is_contiguous() and regions.shape[1] == 2
     for i in range(0, len(slots), 64):
         part = slots[i:i + 64]
