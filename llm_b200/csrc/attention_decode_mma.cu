@@ -36,9 +36,9 @@ int launch_decode_mma(void* out, long long out_stride, const void* q, long long 
   // with one stage, which at head size 64 is also held to 128 registers so that four CTAs share
   // an SM and the grid still runs as one wave where it can (128 requests x 4 kv heads at 640
   // keys: 22.9 us against 28.0 us).
-  // long contexts: about two ranges per SM over all requests (range_length), of a grid that has room for more
+  // long contexts: about two ranges per SM over all requests (ranges_of)
   const int balance = !cluster && max_keys > 2048 ? ranges_at_once(n_kv, llmk_sm_count()) : 0;
-  // (as many CTAs as there can be ranges, see range_length: one wave, or the even share's)
+  // (as many CTAs as there can be ranges: the shares' sum and one for each request that has less than a range's)
   if (balance > 0) grid = dim3((unsigned)((long long)splits * n_entries < balance + n_entries ? splits * n_entries : balance + n_entries), n_kv, 1);
   long long ctas = (long long)splits * n_kv * n_entries;
   if (balance > 0 && ctas > (long long)(balance > n_entries ? balance : n_entries) * n_kv)
@@ -97,15 +97,11 @@ LLMK_API int llmk_decode_attention_ranges(const int* kv_lens, int n_entries, int
                                           int sms, int* ranges) {
   using namespace decode_mma;
   const Mask mask{window, chunk, keep_first};
-  int running = 0;
-  auto over = [&](auto&& count) {
-    int sum = 0;
-    for (int i = 0; i < n_entries; ++i) sum += count(mask.visible(kv_lens[i]));
-    return sum;
-  };
-  LLMK_REQUIRE(n_entries > 0 && n_kv > 0 && splits > 0 && ranges_at_once(n_kv, sms) > 0, "decode_attention_ranges: bad sizes");
-  const int length = range_length(over, splits, ranges_at_once(n_kv, sms), running);
-  for (int i = 0; i < n_entries; ++i) ranges[i] = ranges_of(mask.visible(kv_lens[i]), length, splits);
+  const int balance = n_kv > 0 ? ranges_at_once(n_kv, sms) : 0;
+  LLMK_REQUIRE(n_entries > 0 && splits > 0 && balance > 0, "decode_attention_ranges: bad sizes");
+  int total = 0, running = 0;
+  for (int i = 0; i < n_entries; ++i) total += mask.visible(kv_lens[i]);
+  for (int i = 0; i < n_entries; ++i) running += ranges[i] = ranges_of(mask.visible(kv_lens[i]), total, balance, splits);
   return running * n_kv;
 }
 

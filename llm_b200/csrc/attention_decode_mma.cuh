@@ -101,7 +101,7 @@ __device__ __forceinline__ float2 sum2(const MaybePartial<__nv_bfloat16>& s, siz
 // memory, no fence, no counter.  Every CTA arrives at a first cluster barrier when it starts and waits for it only
 // before it writes to the others, which must be running by then; a second barrier publishes the writes.
 //
-// BALANCE: long contexts, whose ranges are handed out by the requests' lengths (range_length).  A variant of its own, because the code alone,
+// BALANCE: long contexts, whose ranges are handed out by the requests' lengths (ranges_of).  A variant of its own, because the code alone,
 // never run, cost short contexts 0.7 us a launch (64 requests of 600 keys inside a decode step).
 //
 // FUSED: the kernel takes the row of the QKV product itself (a tensor or unsummed split-K
@@ -151,42 +151,16 @@ struct Mask {
 
 // How long contexts are cut: `balance` ranges for all requests together and kv head, as many as run at once, handed out by length, so that
 // one long request among short ones is not walked by as few CTAs as each of them (one of 6,000 keys beside seven of 400, 8 kv heads of
-// 128: four ranges a request 33 us a launch, by length 14.7 us).  All requests get ranges of about one length, the shortest with which they
-// run in one wave.  (Shares rounded to the nearest gave equal requests a piece more than fits: 8 of 8,192 keys, 37 places taken as 5 each, 320
-// CTAs for 296 places, 69 us; 4 each 49 us.  8 of 3,000 33.9 -> 24.5 us; at head size 64, 4 kv heads, 8 of 8,192 24.0 -> 20.6, 10 of 8,192 29.1 ->
-// 24.1, 6,000 beside 400 12.7 -> 10.4; slower: 12 of 300 to 3,600 keys 24.2 -> 25.8, 48 of 4,096 at head size 64 42.5 -> 45.6, where more than one
-// wave of short ranges keeps more bytes in flight.)  Where that length would pass twice the even share, a few long requests are among many
-// short ones, whose places are soon free again, and the even share is taken.  `over` sums a function of the visible keys over the requests;
-// at most `splits` ranges a request; running: the ranges of all of them, at most `balance` plus the number of requests.
-__host__ __device__ inline int ranges_of(int keys, int length, int splits) {
-  const int n = (keys + length - 1) / length;
-  return n < 1 ? 1 : n < splits ? n : splits;      // (an entry without keys: zeros are written)
-}
-template <typename Over>
-__host__ __device__ inline int range_length(Over&& over, int splits, int balance, int& running) {
-  // length 0: the sum of the keys; then the even share, twice that, and by halves to 3 % of it between the two.  (One place that walks the
-  // entries: a launch runs through this code once, so that fetching it is what it costs.)
-  int length = 0, even = 0, fewest = 0, below = 0, fit = 0, at_once = 0;
-  while (true) {
-    const int sum = over([&](int n) { return length ? ranges_of(n, length, splits) : n; });
-    const bool fits = sum <= balance;
-    if (length == 0) {
-      const int share = (sum + balance - 1) / balance;
-      length = even = share > 256 ? share : 256;
-      continue;
-    }
-    if (below == 0) {                                   // the even share
-      if (fits) { running = sum; return even; }
-      fewest = sum;
-      below = even;
-      length = 2 * even;
-      continue;
-    }
-    if (fits) { fit = length; at_once = sum; } else { below = length; }
-    if (fit == 0) { running = fewest; return even; }
-    if ((fit - below) * 32 < even) { running = at_once; return fit; }
-    length = (fit + below) / 2;
-  }
+// 128: four ranges a request 33 us a launch, by length 14.6 us).  A request gets its share of the `total` of all visible keys, rounded down, so that
+// the ranges run in one wave: rounded to the nearest, equal requests got a piece more than fits (8 of 8,192 keys, 37 places taken as 5 each, 320
+// CTAs for 296 places, 69 us; 4 each 47 us; 8 of 3,000 33.9 -> 23.1; at head size 64, 4 kv heads, 8 of 8,192 24.0 -> 19.8, 20 of 4,096 25.2 -> 21.9;
+// slower: 12 of 300 to 3,600 keys 24.2 -> 25.3).  At least one, of at least 256 keys, at most `splits`.  The sum is at most `balance` and one for
+// each request whose share is less than one.  (Lengths found by halving, the shortest with which all ranges run at once, keep ragged requests
+// as even, but eight passes over the lengths before the first key is asked for took more than that gave: 8 of 8,000 keys inside decode steps of
+// 32 layers 4.59 ms a step, this way 4.46.)
+__host__ __device__ inline int ranges_of(int keys, int total, int balance, int splits) {
+  const int share = total > 0 ? (int)((float)keys * (float)balance / (float)total) : 0, most = (keys + 255) / 256 < splits ? (keys + 255) / 256 : splits;
+  return share < 1 || most < 1 ? 1 : share < most ? share : most;      // (an entry without keys: zeros are written)
 }
 
 template <int HS, bool CLUSTER, bool FUSED, bool LIGHT = false, bool EXT = false, bool BALANCE = false>
@@ -235,17 +209,15 @@ decode_attention_mma_kernel(__nv_bfloat16* __restrict__ out, long long out_strid
   int running = (int)(gridDim.x * gridDim.z);                 // ranges of all entries, per kv head
   if constexpr (BALANCE) {
     auto seen_by = [&](int i) { return mask.visible(min(kv_lens[i], table_width * page_size)); };
-    auto over_entries = [&](auto&& count) {
-      int sum = 0;
+    int total = 0;
 #pragma unroll 1
-      for (int i = lane; i < n_entries; i += 32) sum += count(seen_by(i));
-      return __reduce_add_sync(0xffffffffu, sum);
-    };
-    const int length = range_length(over_entries, splits, balance, running);
+    for (int i = lane; i < n_entries; i += 32) total += seen_by(i);
+    total = __reduce_add_sync(0xffffffffu, total);
+    running = max(balance, n_entries);
     e = -1;
 #pragma unroll 1
     for (int i0 = 0, before = 0; i0 < n_entries && e < 0; i0 += 32) {
-      const int own = i0 + lane < n_entries ? ranges_of(seen_by(i0 + lane), length, splits) : 0;
+      const int own = i0 + lane < n_entries ? ranges_of(seen_by(i0 + lane), total, balance, splits) : 0;
       int upto = own;
 #pragma unroll
       for (int o = 1; o < 32; o *= 2) {
