@@ -164,16 +164,10 @@ struct MaybePartial {
   __device__ __forceinline__ bool present() const { return direct != nullptr || parts != nullptr; }
   __device__ __forceinline__ float at(size_t idx) const {
     if (parts) {
-      // loads of eight (then four) splits are issued together; the additions keep the order of the splits
+      // loads of four splits are issued together; the additions keep the order of the splits.  (Eight, with their registers in every consumer:
+      // decode steps of 3 to 16 requests of the routed designs 554 -> 559 and 706 -> 719 us, the others the same.)
       float a = 0.f;
       int s = 0;
-      for (; s + 8 <= splits; s += 8) {
-        float v[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = parts[(size_t)(s + u) * split_stride + idx];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) a += v[u];
-      }
       for (; s + 4 <= splits; s += 4) {
         const float v0 = parts[(size_t)s * split_stride + idx], v1 = parts[(size_t)(s + 1) * split_stride + idx];
         const float v2 = parts[(size_t)(s + 2) * split_stride + idx], v3 = parts[(size_t)(s + 3) * split_stride + idx];
