@@ -1155,18 +1155,19 @@ def _router_logits(h: torch.Tensor, w: torch.Tensor, logits: torch.Tensor, n_tok
     return logits
 
 
-ROUTE_FEW = True      # False: choice, grouping and gather of a step of few tokens are three launches like any other step's
-
-
 @functools.lru_cache(maxsize=None)
-def _moe_few_takes(n_tokens: int, top: int, experts: int) -> bool:
+def moe_route_few_takes(n_tokens: int, top: int, experts: int) -> bool:
+    """Whether one launch can make a step's choices, their grouping and the gather: up to 32 tokens, of which every CTA makes all choices
+    with a warp each."""
     return bool(load().llmk_moe_few_takes(c_int(n_tokens), c_int(top), c_int(experts)))
 
 
-def moe_route_few_takes(n_tokens: int, top: int, experts: int) -> bool:
-    """Whether one launch makes a step's choices, their grouping and the gather: up to 32 tokens, of which every CTA makes all choices
-    with a warp each (7 to 10 us against 10.8 for the three launches of 8 tokens; more tokens than warps would queue)."""
-    return ROUTE_FEW and _moe_few_takes(n_tokens, top, experts)
+def moe_route_few_pays(n_tokens: int, top: int, experts: int, sms: int = 0) -> bool:
+    """Whether that one launch is no slower than the three.  It has a CTA a pair, of up to 1,024 threads, and every CTA makes all choices:
+    beyond a CTA per SM two of them share an SM's schedulers.  Few / three launches, us, the router's product in both: 16 experts, top 4, 8 tokens 7.4 / 11.1, 32
+    tokens 9.8 / 11.9; top 6, 24 tokens (144 pairs) 9.9 / 12.2, 28 tokens (168) 15.0 / 13.3; 32 experts, top 8, 16 tokens 10.8 / 14.2, 32 tokens
+    18.5 / 16.4.  Grouping takes longer with more experts, and from 128 on the one launch stays ahead (top 8, 20 tokens 19.5 / 29.8)."""
+    return moe_route_few_takes(n_tokens, top, experts) and (n_tokens * top <= (sms or sm_count()) or experts >= 128)
 
 
 def moe_route_few(h: torch.Tensor, w: torch.Tensor, bias, logits: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, n_tokens: int, top: int,

@@ -162,7 +162,7 @@ class RoutedFFN(Part):
         gate = ws.flat("moe_shared_gate", ws.max_rows, f32) if self.shared_gate else None
         rows = ws.flat("moe_rows", cap_slots * self.hidden_size, self.dtype).view(cap_slots, self.hidden_size) if tensor else None
         options = dict(over_all=self.over_all, groups=self.groups, gate_out=gate, **self.route_options)
-        if tensor and ops.moe_route_few_takes(T, top, self.outputs):
+        if tensor and ops.moe_route_few_pays(T, top, self.outputs):
             ops.moe_route_few(x, self.w_router, self.b_router, logits, ids, wts, T, top, meta, tile_expert, pair_slot, max_tiles, tile, rows,
                               real=E, **options)
         else:

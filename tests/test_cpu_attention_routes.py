@@ -1,4 +1,4 @@
-"""Which kernel a decode step's attention with options is sent to, on the CPU with the kernels' entry points replaced."""
+"""Which kernels the parts of a decode step are sent to, on the CPU (attention with the kernels' entry points replaced)."""
 import types
 
 import pytest
@@ -25,3 +25,11 @@ def test_chunks_and_sigmoid_weights_beyond_the_counters_take_the_general_kernel(
     group = types.SimpleNamespace(block_table=torch.zeros(entries, 4, dtype=torch.int32))
     ops.paged_attention(q, q, pages, pages, group, ctx, G, G, D, 0, 0.1, **o)
     assert sent == [want]
+
+
+@pytest.mark.parametrize("tokens,top,experts,want", [(8, 4, 16, True), (32, 4, 16, True), (18, 8, 32, True), (19, 8, 32, False), (32, 8, 16, False), (32, 5, 64, False),
+                                                     (20, 8, 128, True), (33, 1, 16, False), (32, 1, 128, False)])
+def test_routing_of_few_tokens_takes_one_launch_while_its_ctas_have_an_sm_each(tokens, top, experts, want):
+    """The last two are more than the launch takes: tokens, or scores in shared memory."""
+    from llm_b200.csrc import ops
+    assert ops.moe_route_few_pays(tokens, top, experts, sms=148) == want
