@@ -26,10 +26,10 @@
 // What bounds it: latency at 16 (eight-warp form) or 8 to 16 warps an SM: half of the issue slots and a fifth of the tensor pipe are in use
 // (what the warps wait for is shared memory and the barriers between a chunk's three parts).  2,048 tokens, the three launches against
 // the token-by-token passes that they took the place of: power form, 8 heads of 128 x 256: 261 -> 132 us; bonus form, 32 heads of
-// 64 x 64: 214 -> 103; scalar form, 32 heads of 128 x 64: 245 -> 74; gate form, 16 heads of 128 x 128: 350 -> 123.  Seven entries of 1
+// 64 x 64: 214 -> 103; scalar form, 32 heads of 128 x 64: 245 -> 76; gate form, 16 heads of 128 x 128: 350 -> 123.  Seven entries of 1
 // to 150 tokens, 8 heads of 32 x 32: 54 -> 39; heads of 8 x 8: 149 -> 39 (the tiles are then mostly padding, and still ahead).
-// Errors against 64 bits (relative, outputs / states): power form 7.8e-7 / 8.7e-7 -> 7.1e-7 / 8.4e-7, bonus form 1.1e-7 / 8.4e-8 ->
-// 1.0e-7 / 6.8e-8, scalar form 1.7e-7 / 1.4e-7 -> 1.7e-7 / 1.3e-7, gate form 1.7e-7 / 3.2e-7 -> 1.6e-7 / 2.8e-7.
+// Errors against 64 bits (relative, outputs / states): power form 7.8e-7 / 8.7e-7 -> 7.4e-7 / 8.4e-7, bonus form 1.1e-7 / 8.4e-8 ->
+// 9.4e-8 / 6.8e-8, scalar form 1.7e-7 / 1.4e-7 -> 1.5e-7 / 1.3e-7, gate form 1.7e-7 / 3.2e-7 -> 1.5e-7 / 2.8e-7.
 #include "diag_chunk.cuh"
 #include "warp_mma.cuh"
 
@@ -43,6 +43,16 @@ constexpr int MAX_SEG = 256;             // tokens of a segment (the scalar form
 
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 __device__ __forceinline__ float log_sigmoid_f(float z) { return fminf(z, 0.f) - log1pf(expf(-fabsf(z))); }
+
+// c += A B, the product in accumulators of its own and the sum a float32 addition.  An MMA that accumulates cuts off what does not fit below
+// its largest term; over the eight steps of 128 channels that was most of the outputs' error (relative to the token-by-token kernel, seven
+// entries of 1 to 150 tokens, eight sets of inputs: gate form of 128 x 128 1.11 with accumulating MMAs, 0.88 this way; bonus form 1.02 and 0.85).
+__device__ __forceinline__ void add_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  float part[4] = {};
+  mma(part, a, b0, b1);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) c[i] += part[i];
+}
 
 // Whether one of eight bfloat16 numbers is infinite or no number.
 __device__ __forceinline__ bool not_finite8(const bf16* p) {
@@ -130,7 +140,7 @@ __device__ void walk_rest(const Args& a, float* rows, int entry, int from, int t
 // of the decays between, which is one number per pair of tokens, and the update's scale stands on v:
 //   o_t = P_t S^T q_t + sum_(s <= t) (q_t . k_s) D_ts v_s,   D_ts = dt_s a_(s+1) .. a_t,     S <- P_C S + sum_s k_s (D_Cs v_s)^T
 // The numbers of a segment (P, D) are made at its start; the scores pass from one MMA's result to the next one's operand in registers.
-// 2,048 tokens, 32 heads of 128 x 64: 155 us for the three launches on the general chunk kernel below, 74 us here.
+// 2,048 tokens, 32 heads of 128 x 64: 155 us for the three launches on the general chunk kernel below, 76 us here.
 template <int DP>
 struct ScalarShape {
   static constexpr int VT = 64, VP = VT + 8, SP = DP + 8, NT = 128;
@@ -232,14 +242,14 @@ scalar_chunk_kernel(const __grid_constant__ Args a) {
         uint32_t qf[4], kf[4];
         ldsm4(qf, q_r + tr * SP + ks * 16 + th);
         ldsm4(kf, k_r + hr * SP + ks * 16 + hh);
-        mma(sc[0], qf, kf[0], kf[1]);
-        mma(sc[1], qf, kf[2], kf[3]);
+        add_mma(sc[0], qf, kf[0], kf[1]);
+        add_mma(sc[1], qf, kf[2], kf[3]);
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
           uint32_t b0[3], b1[3];
           split3(st[2 * ks][2 * nt], st[2 * ks][2 * nt + 1], b0);
           split3(st[2 * ks + 1][2 * nt], st[2 * ks + 1][2 * nt + 1], b1);
-          mma(hi[nt], qf, b0[0], b1[0]);
+          add_mma(hi[nt], qf, b0[0], b1[0]);
           mma(lo[nt], qf, b0[1], b1[1]);
           mma(lo[nt], qf, b0[2], b1[2]);
         }
@@ -595,7 +605,7 @@ diag_chunk_kernel(const __grid_constant__ Args a) {
           uint32_t b0[3], b1[3];
           split3(st[2 * ks][2 * nt], st[2 * ks][2 * nt + 1], b0);
           split3(st[2 * ks + 1][2 * nt], st[2 * ks + 1][2 * nt + 1], b1);
-          mma(hi[nt], qf[0], b0[0], b1[0]);
+          add_mma(hi[nt], qf[0], b0[0], b1[0]);
           mma(lo[nt], qf[0], b0[1], b1[1]);
           mma(lo[nt], qf[1], b0[0], b1[0]);
           mma(lo[nt], qf[0], b0[2], b1[2]);
