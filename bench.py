@@ -344,8 +344,9 @@ def decode_attention_sweep(args, peaks, torch, ops) -> int:
         kv_lens = torch.full((batch,), ctx, dtype=torch.int32, device=dev)
         q = torch.randn(batch, n_heads * hs, device=dev, dtype=torch.bfloat16)
         out = torch.empty_like(q)
+        splits = ops.decode_places(batch, n_kv * args.head_parts, ctx)      # as the engine asks for them
         call = lambda i: ops.paged_attention_decode(out, q, k_pages, v_pages, tables[i % sets], kv_lens, batch, n_heads, n_kv,
-                                                    hs, 0, 1.0 / math.sqrt(hs), max_keys=ctx, head_parts=args.head_parts)
+                                                    hs, 0, 1.0 / math.sqrt(hs), splits=splits, max_keys=ctx, head_parts=args.head_parts)
         for i in range(3):
             call(i)
         torch.cuda.synchronize()
@@ -361,7 +362,7 @@ def decode_attention_sweep(args, peaks, torch, ops) -> int:
         torch.cuda.synchronize()
         us = a.elapsed_time(b) / n * 1e3
         gbs = nbytes / us / 1e3
-        print(f"batch {batch:3d} context {ctx:6d} ranges {ops.decode_splits(batch, n_kv, ctx):2d}: {us:8.1f} us a launch, "
+        print(f"batch {batch:3d} context {ctx:6d} ranges {ops.decode_splits(batch, n_kv * args.head_parts, ctx):2d}: {us:8.1f} us a launch, "
               f"{nbytes / 1e6:7.1f} MB, {gbs:7.1f} GB/s = {gbs / peaks['hbm_gbs']:.2f} of the peak")
         del k_pages, v_pages, tables
     return 0

@@ -136,7 +136,8 @@ namespace {
 // the values are the keys as projected, before norm and rotation (vdim = dim).
 // VEC: four channels at a time (dim and the rows on the 4-grid).  A few tokens are bound by the loads of their partial results (eight
 // of a channel, a round trip to L2 for every four), so a CTA of 512 threads has a row of 2,560 channels in flight at once, and the angles
-// are made once per CTA: 8 tokens, 20 heads of 128, 18.9 -> 8.3 us a launch inside a decode step.
+// are made once per CTA: 8 tokens, 20 heads of 128, 18.9 -> 8.3 us a launch inside a decode step.  (With 256 and 512 threads, us: 16 tokens 6.5
+// and 5.1, 128 tokens 7.4 and 6.4, 256 tokens 9.8 and 7.0, 512 tokens 11.7 and 12.7: 512 up to 128 tokens.)
 // Shared memory: the row, rounded up to whole pairs of floats, then a cosine and a sine per pair that turns (`table`), unless a row
 // and angles of that size do not fit together: every pair then makes its own.
 constexpr size_t NORM_ROPE_SMEM = 226 * 1024;      // of the 227 KB of a CTA; the sums' scratch takes 128 bytes

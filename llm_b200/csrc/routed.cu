@@ -422,7 +422,8 @@ struct CombineMore {
 // four columns per thread where the rows allow 16-byte loads
 // AHEAD (few tokens): the rows of four pairs are asked for before the first is used, the shared expert's row and the result go four columns
 // at once (16 tokens, split-K partial results, inside a decode step: 5.9 -> 3.8 us); with many tokens there are warps enough, which
-// its registers cost (2,048 tokens, four pairs each: 13.3 us without, 15.7 us with it).
+// its registers cost (four pairs each, without and with it: 128 tokens 2.6 and 2.5 us, with split-K partial results 5.1 and 3.1; 512 tokens 4.1 and
+// 4.2, 8.4 and 5.7; 2,048 tokens 13.3 and 15.7).
 template <typename T, bool AHEAD>
 __global__ void combine4_kernel(T* __restrict__ out, const float* __restrict__ y, const int* __restrict__ pair_slot,
                                 const float* __restrict__ weights, MaybePartial<T> shared, int top, int width, size_t total4,

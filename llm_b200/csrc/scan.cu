@@ -469,7 +469,7 @@ pair_norm_mean_kernel(T* __restrict__ out, MaybePartial<T> a, MaybePartial<T> b,
   float sa = 0.f, sb = 0.f;
   if (VEC) {
     // four columns a thread, so that all partial results of a row of 2,048 are in flight at once (8 tokens inside a decode step, a column
-    // at a time: 12.3 us, this way 6.9 us)
+    // at a time: 12.3 us, this way 6.9 us; with 256 and 512 threads: 16 tokens 8.4 and 5.2, 128 tokens 8.6 and 6.3, 512 tokens 13.6 and 12.5)
     for (int c = threadIdx.x * 4; c < width; c += blockDim.x * 4) {
       float va[4], vb[4];
       a.at4(base + c, va);
