@@ -97,6 +97,78 @@ gemm_simt_kernel(const T* __restrict__ A, const T* __restrict__ W, TC* __restric
   }
 }
 
+// Products too small for the tiles above to fill the chip (float32, 16-byte pieces): tiles of 16 x 32, the whole of K (in blocks of 128, two of
+// them in flight) asked for at once instead of 16 k at a time behind two barriers.  Each element is one chain of multiply-adds over k = 0..K-1,
+// as above, so that a product's bits do not depend on which of the two kernels made it.  The weights of the first blocks are asked for
+// before the kernel waits.  Both are bound by latency at these sizes, and a 64 x 64 tile on one SM also takes 4 us of multiply-adds at K = 256:
+// in the steps of a model of width 96 (feed-forward 256, up to 100 rows) a launch took 8.2 us with the large tiles, 3.0 us with these.
+constexpr int SBM = 16, SBN = 32, SBK = 128, SPITCH = SBK + 4;
+
+__global__ void __launch_bounds__(128)
+gemm_simt_small_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K, long long lda,
+                       long long ldw, long long ldc, long long a_batch, long long w_batch, long long c_batch,
+                       const float* __restrict__ gate, long long gate_stride) {
+  extern __shared__ __align__(16) float tiles[];          // [2][SBM + SBN][SPITCH]
+  pdl_launch_dependents();
+  const int tid = threadIdx.x, m0 = blockIdx.y * SBM, n0 = blockIdx.x * SBN;
+  A += (size_t)blockIdx.z * a_batch;
+  W += (size_t)blockIdx.z * w_batch;
+  C += (size_t)blockIdx.z * c_batch;
+  // a thread copies its 16 bytes (four k) of every fourth row; rows past the end give results that nobody stores
+  const int copy_k = (tid & 31) * 4, copy_row = tid >> 5;
+  auto copy = [&](int block, const float* src, long long ld, int rows, int row0, int first, int last) {
+    const int k = block * SBK + copy_k;
+    if (k >= K) return;
+    float* dst = tiles + ((size_t)(block & 1) * (SBM + SBN) + first) * SPITCH + copy_k;
+    for (int r = copy_row; r < last; r += 4)
+      if (row0 + r < rows) cp_async16(dst + r * SPITCH, src + (size_t)(row0 + r) * ld + k);
+  };
+  auto commit = []() { asm volatile("cp.async.commit_group;" ::: "memory"); };
+  const int blocks = (K + SBK - 1) / SBK;
+  copy(0, W, ldw, N, n0, SBM, SBN);
+  if (blocks > 1) copy(1, W, ldw, N, n0, SBM, SBN);
+  pdl_wait();
+  copy(0, A, lda, M, m0, 0, SBM);
+  commit();
+  if (blocks > 1) copy(1, A, lda, M, m0, 0, SBM);
+  commit();
+  const int m = (tid >> 4) * 2, n = tid & 15;              // this thread's elements: rows m, m + 1, columns n, n + 16
+  float acc[2][2] = {};
+  for (int b = 0; b < blocks; ++b) {
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    const float* a = tiles + ((size_t)(b & 1) * (SBM + SBN) + m) * SPITCH;
+    const float* w = tiles + ((size_t)(b & 1) * (SBM + SBN) + SBM + n) * SPITCH;
+    const int here = min(SBK, K - b * SBK);
+#pragma unroll 4
+    for (int k = 0; k < here; k += 4) {
+      float x[2][4], y[2][4];
+      Vec4<float>::load(a + k, x[0]); Vec4<float>::load(a + SPITCH + k, x[1]);
+      Vec4<float>::load(w + k, y[0]); Vec4<float>::load(w + 16 * SPITCH + k, y[1]);
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) acc[i][j] = fmaf(x[i][kk], y[j][kk], acc[i][j]);
+    }
+    if (b + 2 < blocks) {
+      __syncthreads();
+      copy(b + 2, W, ldw, N, n0, SBM, SBN);
+      copy(b + 2, A, lda, M, m0, 0, SBM);
+    }
+    commit();
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    if (m0 + m + i >= M) continue;
+    const float g = gate ? 1.f / (1.f + expf(-gate[(size_t)(m0 + m + i) * gate_stride + blockIdx.z])) : 1.f;
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      if (n0 + n + 16 * j < N) C[(size_t)(m0 + m + i) * ldc + n0 + n + 16 * j] = gate ? acc[i][j] * g : acc[i][j];
+  }
+}
+
 template <typename T, typename TC>
 int launch(const void* A, const void* W, void* C, int M, int N, int K, long long lda, long long ldw,
            long long ldc, cudaStream_t stream, int batches = 1, long long a_batch = 0, long long w_batch = 0,
@@ -104,6 +176,17 @@ int launch(const void* A, const void* W, void* C, int M, int N, int K, long long
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batches);
   const bool vec = (K % 4 == 0) && (lda % 4 == 0) && (ldw % 4 == 0) && (a_batch % 4 == 0) && (w_batch % 4 == 0) &&
                    ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
+  if constexpr (sizeof(T) == 4 && sizeof(TC) == 4) {
+    // the small tiles while the large ones would leave more than half of the SMs idle
+    if (vec && (long long)grid.x * grid.y * grid.z * 2 <= llmk_sm_count()) {
+      const size_t smem = 2 * (SBM + SBN) * SPITCH * sizeof(float);
+      cudaError_t e = cudaFuncSetAttribute(gemm_simt_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return llmk_fail((int)e, "gemm_simt: %s", cudaGetErrorString(e));
+      launch_kernel(gemm_simt_small_kernel, dim3((N + SBN - 1) / SBN, (M + SBM - 1) / SBM, batches), dim3(128), smem, stream, (const float*)A,
+                    (const float*)W, (float*)C, M, N, K, lda, ldw, ldc, a_batch, w_batch, c_batch, (const float*)gate, gate_stride);
+      LLMK_LAUNCH_CHECK("gemm_simt_small");
+    }
+  }
   if (vec)
     launch_kernel(gemm_simt_kernel<T, TC, 4>, grid, dim3(THREADS), 0, stream, (const T*)A, (const T*)W, (TC*)C, M, N, K, lda, ldw, ldc,
                   a_batch, w_batch, c_batch, (const T*)gate, gate_stride);
