@@ -24,7 +24,12 @@
 namespace {
 
 constexpr int WARPS = 4;
-constexpr int MAX_HEAD_DIM = 1024;     // the kernel is built for head sizes up to 256, up to 512 and up to 1024
+// The kernel is built for head sizes up to 64, 128, 256, 512 and 1024: a lane walks over MAXD / 32 channels of every key, whether the head has
+// them or not, and with one warp on a scheduler each of these instructions costs its latency.  (Head size 32, up to 113 keys, float32, inside
+// decode steps of four requests: 29.0 us a launch when the smallest build was 256 and a key's values were loaded one key after the other;
+// 18.3 us this way, with the rows asked for ahead.)
+constexpr int MAX_HEAD_DIM = 1024;
+constexpr int PREFETCH_TILES = 4;      // tiles of keys and values asked into L1 ahead of their turn
 
 template <typename T>
 __device__ __forceinline__ float dot_row(const float* __restrict__ q, const T* __restrict__ k, int head_dim);
@@ -33,6 +38,7 @@ template <>
 __device__ __forceinline__ float dot_row<float>(const float* __restrict__ q, const float* __restrict__ k,
                                                 int head_dim) {
   float s = 0.f;
+#pragma unroll 8
   for (int d = 0; d < head_dim; d += 4) {
     const float4 kv = *reinterpret_cast<const float4*>(k + d);
     s = fmaf(q[d], kv.x, s);
@@ -79,6 +85,7 @@ paged_attention_generic_kernel(T* __restrict__ out, long long out_stride, const 
                                float softcap, int sink, bool vec, const float* __restrict__ sink_values, int chunk,
                                const float* __restrict__ sigmoid_bias, const float* __restrict__ dist_r1,
                                const float* __restrict__ dist_r2, int v_share) {
+  constexpr int AHEAD = MAXD <= 256 ? 8 : MAXD <= 512 ? 4 : 2;
   __shared__ float q_s[WARPS][MAXD];
   pdl_launch_dependents();      // let the next kernel start its own prologue now
   pdl_wait();
@@ -100,6 +107,20 @@ paged_attention_generic_kernel(T* __restrict__ out, long long out_stride, const 
   for (int d = lane; d < head_dim; d += 32) q_s[warp][d] = to_f32(q_row[d]);
   __syncwarp();
 
+  // a tile's page number, keys and values follow from one another, three trips to L2: short rows are asked for some tiles ahead
+  auto prefetch_tile = [&](int tile) {
+    const int kp = tile + lane;
+    if (kp > pos || kp < lo) return;
+    const int page = table[kp / page_size], at = kp % page_size;
+    const char* k = reinterpret_cast<const char*>(k_pages + (((long long)page * n_kv + g) * page_size + at) * head_dim);
+    const char* v = reinterpret_cast<const char*>(v_pages + (((long long)page * n_v + gv) * page_size + at) * vdim);
+    for (int b = 0; b < head_dim * (int)sizeof(T); b += 128) asm volatile("prefetch.global.L1 [%0];" ::"l"(k + b));
+    for (int b = 0; b < vdim * (int)sizeof(T); b += 128) asm volatile("prefetch.global.L1 [%0];" ::"l"(v + b));
+  };
+  const bool ahead = MAXD <= 64 && keep_end == 0;
+  if (ahead)
+    for (int i = 0; i < PREFETCH_TILES; ++i) prefetch_tile(lo_tile + 32 * i);
+
   float acc[MAXD / 32];
 #pragma unroll
   for (int i = 0; i < MAXD / 32; ++i) acc[i] = 0.f;
@@ -113,6 +134,7 @@ paged_attention_generic_kernel(T* __restrict__ out, long long out_stride, const 
       tile = lo_tile - 32;
       continue;
     }
+    if (ahead) prefetch_tile(tile + 32 * PREFETCH_TILES);
     const int kp = tile + lane;
     const bool valid = kp <= pos && (kp >= lo || kp < keep_end);
     long long row = 0;                             // the value's place in units of rows of vdim
@@ -137,18 +159,23 @@ paged_attention_generic_kernel(T* __restrict__ out, long long out_stride, const 
 #pragma unroll
       for (int i = 0; i < MAXD / 32; ++i) acc[i] *= alpha;
     }
+    // the values of several keys asked for together (a key after the other waits for memory 32 times a tile), added in the keys' order
     const int n_valid = min(32, pos - tile + 1);
-    for (int j = 0; j < n_valid; ++j) {
-      const float pj = __shfl_sync(0xffffffffu, p, j);
-      const long long rj = __shfl_sync(0xffffffffu, row, j);
-      if (pj != 0.f) {
-        const T* v = v_pages + rj * vdim;
+#pragma unroll 1
+    for (int j = 0; j < n_valid; j += AHEAD) {
+      float v[AHEAD][MAXD / 32], pj[AHEAD];
 #pragma unroll
-        for (int i = 0; i < MAXD / 32; ++i) {
-          const int d = lane + 32 * i;
-          if (d < vdim) acc[i] = fmaf(pj, to_f32(v[d]), acc[i]);
-        }
+      for (int u = 0; u < AHEAD; ++u) {
+        pj[u] = __shfl_sync(0xffffffffu, p, j + u);            // 0 for a key past the last (AHEAD divides 32)
+        const T* at = v_pages + __shfl_sync(0xffffffffu, row, j + u) * vdim;
+#pragma unroll
+        for (int i = 0; i < MAXD / 32; ++i) v[u][i] = pj[u] != 0.f && lane + 32 * i < vdim ? to_f32(at[lane + 32 * i]) : 0.f;
       }
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u)
+        if (pj[u] != 0.f)
+#pragma unroll
+          for (int i = 0; i < MAXD / 32; ++i) acc[i] = fmaf(pj[u], v[u][i], acc[i]);
     }
   }
   const float inv = gated ? 1.f : 1.f / l;
@@ -194,21 +221,14 @@ LLMK_API int llmk_paged_attention_generic_ex(void* out, long long out_stride, co
   return dispatch_dtype(dtype, [&](auto* tag) {
     using T = LLMK_ELEM(tag);
     const bool vec = head_dim % (16 / (int)sizeof(T)) == 0 && (uintptr_t)k_pages % 16 == 0;      // whole 16-byte pieces per key row
-    if (widest <= 256)
-      launch_kernel(paged_attention_generic_kernel<T, 256>, dim3((unsigned)blocks), dim3(WARPS * 32), 0, stream,
-          (T*)out, out_stride, (const T*)q, q_stride, (const T*)k_pages, (const T*)v_pages, block_table,
-          table_width, token_entry, positions, n_tokens, n_heads, n_kv, head_dim, vdim, page_size, window, keep_first, scale,
-          softcap, sink, vec, sink_values, chunk, sigmoid_bias, dist_r1, dist_r2, v_share);
-    else if (widest <= 512)      // the wide head of a latent attention (its rank)
-      launch_kernel(paged_attention_generic_kernel<T, 512>, dim3((unsigned)blocks), dim3(WARPS * 32), 0, stream,
-          (T*)out, out_stride, (const T*)q, q_stride, (const T*)k_pages, (const T*)v_pages, block_table,
-          table_width, token_entry, positions, n_tokens, n_heads, n_kv, head_dim, vdim, page_size, window, keep_first, scale,
-          softcap, sink, vec, sink_values, chunk, sigmoid_bias, dist_r1, dist_r2, v_share);
-    else
-      launch_kernel(paged_attention_generic_kernel<T, MAX_HEAD_DIM>, dim3((unsigned)blocks), dim3(WARPS * 32), 0, stream,
-          (T*)out, out_stride, (const T*)q, q_stride, (const T*)k_pages, (const T*)v_pages, block_table,
-          table_width, token_entry, positions, n_tokens, n_heads, n_kv, head_dim, vdim, page_size, window, keep_first, scale,
-          softcap, sink, vec, sink_values, chunk, sigmoid_bias, dist_r1, dist_r2, v_share);
+    auto kern = widest <= 64 ? paged_attention_generic_kernel<T, 64> : widest <= 128 ? paged_attention_generic_kernel<T, 128>
+                : widest <= 256 ? paged_attention_generic_kernel<T, 256>
+                : widest <= 512 ? paged_attention_generic_kernel<T, 512>      // the wide head of a latent attention (its rank)
+                : paged_attention_generic_kernel<T, MAX_HEAD_DIM>;
+    launch_kernel(kern, dim3((unsigned)blocks), dim3(WARPS * 32), 0, stream,
+        (T*)out, out_stride, (const T*)q, q_stride, (const T*)k_pages, (const T*)v_pages, block_table,
+        table_width, token_entry, positions, n_tokens, n_heads, n_kv, head_dim, vdim, page_size, window, keep_first, scale,
+        softcap, sink, vec, sink_values, chunk, sigmoid_bias, dist_r1, dist_r2, v_share);
     LLMK_LAUNCH_CHECK("paged_attention_generic");
   });
 }
