@@ -29,7 +29,7 @@ GROUPS = {
                          "attention_decode.cu", "sampling.cu", "latent.cu", "routed.cu", "recurrent.cu", "diag_chunk.cu", "hyper.cu",
                          "short_conv.cu", "scan.cu", "delta.cu", "lightning.cu", "mlstm.cu",
                          "sandwich.cu"]),
-    "tensor": ("libllm_b200_tensor.so", ["runtime.cu", "gemm_tc.cu", "attention_tc.cu", "attention_decode_mma.cu", "attention_wide.cu"]),
+    "tensor": ("libllm_b200_tensor.so", ["runtime.cu", "gemm_tc.cu", "gemm_few.cu", "attention_tc.cu", "attention_decode_mma.cu", "attention_wide.cu"]),
     # host side of the runtime (page pool, step metadata, scheduler): plain C++, built with g++, needs no CUDA
     "host": ("libllm_b200_host.so", ["host/page_pool.cpp", "host/scheduler.cpp"]),
 }

@@ -62,6 +62,13 @@ class WeightedRows:
         self.shared, self.shared_gate, self.ids, self.first_identity, self.x = shared, shared_gate, ids, first_identity, x
 
 
+class NormedRows:
+    """rms(resid[:rows]) * gain, still to be formed by the product that reads it (gemm_few) from float32 rows of a residual stream."""
+
+    def __init__(self, resid: torch.Tensor, gain: torch.Tensor, eps: float, rows: int, dtype: torch.dtype):
+        self.resid, self.gain, self.eps, self.rows, self.dtype = resid, gain, eps, rows, dtype
+
+
 def _split_args(x):
     """(direct pointer, partials pointer, splits, split stride) of a tensor, a PartialSum or None."""
     if isinstance(x, PartialSum):
@@ -1978,6 +1985,57 @@ def gemm_fast(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, rows: int, pl
     _check_t(lib.llmk_reduce_partials(_ptr(out), _ptr(part), c_longlong(rows * n), c_int(splits),
                                     c_int(_kind(out.dtype)), _stream()))
     return out
+
+
+GEMM_FEW = True
+FEW_ROWS = 8
+_FEW_SMEM = 227 * 1024
+_FEW_KINDS = {"add": 2, "silu": 3, "relu": 4}
+
+
+@functools.lru_cache(maxsize=4096)
+def gemm_few_takes(rows: int, k: int) -> bool:
+    """Whether the few-row product takes so many rows of k channels (as llmk_gemm_few_supported)."""
+    rest = k * rows * 2 + 4 * k + 2 * 8 * 160 * 4 + 256 + 33 * 8
+    return 0 < rows <= FEW_ROWS and k > 0 and k % 64 == 0 and rest + 3 * 16384 <= _FEW_SMEM
+
+
+def gemm_few_available(a, w: torch.Tensor, rows: int) -> bool:
+    """Whether gemm_few takes these operands: bfloat16 (or NormedRows), few rows, 16-byte aligned."""
+    if not GEMM_FEW or w.dtype != torch.bfloat16 or not gemm_few_takes(rows, w.shape[1]) or w.stride(0) % 8 or w.data_ptr() % 16 or not w.is_cuda:
+        return False
+    if isinstance(a, NormedRows):
+        return True
+    return a.dtype == torch.bfloat16 and a.is_cuda and a.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0
+
+
+def gemm_few(a, w: torch.Tensor, out: torch.Tensor, rows: int, kind=None) -> torch.Tensor:
+    """out[:rows] = a[:rows] @ w.T for up to 8 rows (gemm_few.cu): every output is one sum, nothing is left to be added up.  a: bfloat16
+    rows or NormedRows.  kind None: written in out's dtype; "add": added to float32 out; "silu" or "relu": w = [gate; up] stacked,
+    act(a @ gate.T) * (a @ up.T) in bfloat16."""
+    _rows_contig(w, "w"); _rows_contig(out, "out")
+    n, k = w.shape
+    n = n // 2 if kind in ("silu", "relu") else n
+    assert out.shape[1] == n and out.shape[0] >= rows and (kind is None or out.dtype == (torch.float32 if kind == "add" else torch.bfloat16))
+    if isinstance(a, NormedRows):
+        assert a.resid.dtype == a.gain.dtype == torch.float32 and a.resid.shape[1] == k == a.gain.numel() and rows == a.rows
+        _rows_contig(a.resid, "rows")
+        src = (c_void_p(0), _ptr(a.resid), _ptr(a.gain), c_float(a.eps), c_longlong(a.resid.stride(0)))
+    else:
+        _rows_contig(a, "a")
+        assert a.shape[1] == k and a.dtype == torch.bfloat16
+        src = (_ptr(a), c_void_p(0), c_void_p(0), c_float(0.0), c_longlong(a.stride(0)))
+    code = _FEW_KINDS[kind] if kind else int(out.dtype == torch.bfloat16)
+    _check_t(load_tensor().llmk_gemm_few(*src, _ptr(w), c_longlong(w.stride(0)), _ptr(out), c_longlong(out.stride(0)), c_int(rows), c_int(n),
+                                         c_int(k), c_int(code), _stream()))
+    return out
+
+
+def gemm_few_sums(a, w: torch.Tensor, rows: int, dtype: torch.dtype) -> PartialSum:
+    """a[:rows] @ w.T as a PartialSum of one term: float32 sums for a kernel that takes one, with nothing rounded in between."""
+    part = _partials(w.device)
+    gemm_few(a, w, part[:rows * w.shape[0]].view(rows, w.shape[0]), rows)
+    return PartialSum(part, 1, rows, w.shape[0], dtype)
 
 
 def gemm_swiglu_available(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, rows: int) -> bool:

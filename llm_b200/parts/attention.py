@@ -32,7 +32,7 @@ import torch
 
 from ..csrc import ops
 from .base import CacheNeed, ParamInfo, Part, StateNeed, build_part, register_part
-from .linear import FUSE_PARTIALS, linear
+from .linear import FUSE_PARTIALS, linear, linear_add
 
 
 _NAMES = {"q": "q_proj.weight", "k": "k_proj.weight", "v": "v_proj.weight", "o": "o_proj.weight",
@@ -192,11 +192,14 @@ class PagedAttention(Part):
         # then measured best (64 requests: 1.29 ms a step with a third, 1.20 ms with half or all)
         return ops.sm_count() // (2 if ctx.n_tokens >= ops.NORMAL_MODE_FROM_ROWS else 3)
 
-    def forward(self, x: torch.Tensor, ctx, view) -> torch.Tensor:
+    def reads_unformed(self, rows, ctx) -> bool:
+        return not self.extended and ops.gemm_few_available(rows, self.w_qkv, ctx.n_tokens)
+
+    def forward(self, x: torch.Tensor, ctx, view, into=None):
         T = ctx.n_tokens
         ws = ctx.workspace
         if self.extended:
-            return self._forward_extended(x, ctx, view)
+            return self._forward_extended(x, ctx, view, into)
         width = self.q_size + 2 * self.kv_size
         cos = sin = None
         own_transform = None
@@ -233,11 +236,13 @@ class PagedAttention(Part):
                               k_pages.shape[1], self.head_dim, self.window or 0, self.scale,
                               write_kv=not self.shares_cache,
                               q_rot=lambda: ws.get("q_rot", T, self.q_size, self.dtype))
+        if into is not None and self.b_o is None and linear_add(attn, self.w_o, into.resid, T):
+            return None
         return linear(attn, self.w_o, ws.get("mixer_out", T, self.hidden_size, self.dtype), T, allow_partial=FUSE_PARTIALS,
                       bias=self.b_o)
 
 
-    def _forward_extended(self, x: torch.Tensor, ctx, view) -> torch.Tensor:
+    def _forward_extended(self, x: torch.Tensor, ctx, view, into=None):
         """One product for q, k, v (its split-K partial results go unsummed to the next kernel); one kernel that
         sums them, turns the pairs of q and k and stores k and v in the pages; the attention kernel that takes
         the options; the output projection."""
@@ -267,6 +272,8 @@ class PagedAttention(Part):
                             value_dim=V, softcap=self.softcap, sink=self.sink, keep_first=self.keep_first,
                             chunk=self.chunk, sigmoid_bias=self.score_bias, sink_values=self.sink_values,
                             dist_bias=(self.r1, self.r2) if self.dist_bias else None)
+        if into is not None and linear_add(attn, self.w_o, into.resid, T):
+            return None
         return linear(attn, self.w_o, ws.get("mixer_out", T, self.hidden_size, self.dtype), T, allow_partial=FUSE_PARTIALS)
 
 

@@ -8,6 +8,7 @@ out norm2 and ffn: it is x += mixer(norm1(x)) alone.
 from __future__ import annotations
 
 import dataclasses
+import inspect
 
 import torch
 
@@ -27,6 +28,9 @@ class PreNormBlock:
                       for r in self.roles}
         self.norm1, self.mixer = self.parts["norm1"], self.parts["mixer"]
         self.norm2, self.ffn = self.parts["norm2"], self.parts["ffn"]
+        # a part whose forward takes `into` may read rows before their norm and add its result to the stream itself
+        takes = lambda part: part is not None and "into" in inspect.signature(part.forward).parameters
+        self.mixer_into, self.ffn_into = takes(self.mixer), takes(self.ffn)
         # a feed-forward that keeps something per request (the inputs of a convolution over time) says so with state_need();
         # the layer's state row is then the mixer's numbers followed by the feed-forward's
         self.ffn_state = self.ffn.state_need() if self.ffn is not None and hasattr(self.ffn, "state_need") else None
@@ -46,11 +50,23 @@ class PreNormBlock:
             return self.mixer.state_need()
         return StateNeed((self.mixer_cols + int(self.ffn_state.shape[0]),), torch.float32)
 
+    @staticmethod
+    def _rows(norm, part, takes_into: bool, stream: ResidualStream, ctx):
+        """What the sublayer reads: the normed rows, or, where its first product can norm what it reads, the rows before their norm."""
+        if takes_into and hasattr(norm, "unformed") and hasattr(part, "reads_unformed"):
+            rows = norm.unformed(stream)
+            if rows is not None and part.reads_unformed(rows, ctx):
+                return rows
+        return norm.forward(stream, ctx)
+
     def forward(self, stream: ResidualStream, ctx, view) -> None:
         if self.ffn_state is None:
-            stream.pending = self.mixer.forward(self.norm1.forward(stream, ctx), ctx, view)
+            # a sublayer whose last product can add to the stream does so (and returns None), else its result is left pending
+            into = {"into": stream} if self.mixer_into else {}
+            stream.pending = self.mixer.forward(self._rows(self.norm1, self.mixer, self.mixer_into, stream, ctx), ctx, view, **into)
             if self.ffn is not None:
-                stream.pending = self.ffn.forward(self.norm2.forward(stream, ctx), ctx)
+                into = {"into": stream} if self.ffn_into else {}
+                stream.pending = self.ffn.forward(self._rows(self.norm2, self.ffn, self.ffn_into, stream, ctx), ctx, **into)
             return
         rows = view.state.view(view.state.shape[0], -1)
         mixer_view = dataclasses.replace(view, state=rows[:, :self.mixer_cols] if self.mixer_cols else None)

@@ -22,7 +22,7 @@ import torch
 
 from ..csrc import ops
 from .base import CacheNeed, ParamInfo, Part, register_part
-from .linear import FUSE_PARTIALS, linear
+from .linear import FUSE_PARTIALS, linear, linear_add
 
 _NAMES = {"q": "q", "k": "k", "v": "v", "gate": "g", "out": "o", "q_norm": "q.norm", "k_norm": "k.norm",
           "lq1": "lq1", "lk1": "lk1", "lq2": "lq2", "lk2": "lk2"}
@@ -78,7 +78,7 @@ class DifferentialAttention(Part):
     def state_need(self):
         return None
 
-    def forward(self, x: torch.Tensor, ctx, view) -> torch.Tensor:
+    def forward(self, x: torch.Tensor, ctx, view, into=None):
         T, ws = ctx.n_tokens, ctx.workspace
         H, G, D, V = self.num_heads, self.num_kv_heads, self.head_dim, self.value_dim
         width = self.q_size + self.k_size + self.v_size + (self.o_size if self.gated else 0)
@@ -92,6 +92,8 @@ class DifferentialAttention(Part):
         gate = proj[:, self.q_size + self.k_size + self.v_size:] if self.gated else None
         out = ws.get("attn_out", T, self.o_size, self.dtype)
         ops.diff_combine(out, maps, gate, T, H, self.per_group, self.lam, 1.0 - self.diff, self.eps)
+        if into is not None and linear_add(out, self.w_o, into.resid, T):
+            return None
         return linear(out, self.w_o, ws.get("mixer_out", T, self.hidden_size, self.dtype), T, allow_partial=FUSE_PARTIALS)
 
 

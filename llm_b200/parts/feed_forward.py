@@ -11,7 +11,7 @@ import torch
 
 from ..csrc import ops
 from .base import ParamInfo, Part, register_part
-from .linear import FUSE_PARTIALS, linear, linear_act, linear_swiglu
+from .linear import FUSE_PARTIALS, linear, linear_act, linear_add, linear_swiglu
 
 
 _GLU_NAMES = {"gate": "gate_proj.weight", "up": "up_proj.weight", "down": "down_proj.weight",
@@ -58,14 +58,19 @@ class SwiGLU(Part):
             self.b_gate_up = torch.cat([n("gate_bias"), n("up_bias")]).contiguous()
             self.b_down = n("down_bias").contiguous()
 
-    def forward(self, x: torch.Tensor, ctx, tag: str = "ffn") -> torch.Tensor:
+    def reads_unformed(self, rows, ctx) -> bool:
+        return ops.gemm_few_available(rows, self.w_gate_up, ctx.n_tokens)
+
+    def forward(self, x: torch.Tensor, ctx, tag: str = "ffn", into=None):
         T, ws = ctx.n_tokens, ctx.workspace
         act = ws.get(tag + "_act", T, self.intermediate_size, self.dtype)
-        # with many rows the product's epilogue makes the activation; with few rows, or biases, the row kernel
+        # the product's epilogue makes the activation; where K is split over CTAs, or with biases, the row kernel
         if self.bias or not linear_swiglu(x, self.w_gate_up, act, T, self.activation):
             gate_up = linear(x, self.w_gate_up, ws.get("gate_up", T, 2 * self.intermediate_size, self.dtype), T,
                              allow_partial=FUSE_PARTIALS, bias=self.b_gate_up)
             ops.silu_mul(act, gate_up, T, self.activation)
+        if into is not None and self.b_down is None and linear_add(act, self.w_down, into.resid, T):
+            return None
         return linear(act, self.w_down, ws.get(tag + "_out", T, self.hidden_size, self.dtype), T, allow_partial=FUSE_PARTIALS,
                       bias=self.b_down)
 
@@ -109,7 +114,7 @@ class ActMLP(Part):
             self.b_up = tensors[self.name(self.up_name + ".b")].contiguous()
             self.b_down = tensors[self.name(self.down_name + ".b")].contiguous()
 
-    def forward(self, x: torch.Tensor, ctx, tag: str = "ffn", allow_unsummed: bool = False):
+    def forward(self, x: torch.Tensor, ctx, tag: str = "ffn", allow_unsummed: bool = False, into=None):
         T, ws = ctx.n_tokens, ctx.workspace
         act = ws.get(tag + "_act", T, self.intermediate_size, self.dtype)
         if self.bias:
@@ -123,6 +128,8 @@ class ActMLP(Part):
         if not linear_act(x, self.w_up, act, T, self.activation):      # many rows: the activation in the product's epilogue
             up = linear(x, self.w_up, ws.get(tag + "_up", T, self.intermediate_size, self.dtype), T, allow_partial=FUSE_PARTIALS)
             ops.act_rows(act, up, T, self.activation)
+        if into is not None and linear_add(act, self.w_down, into.resid, T):
+            return None
         return linear(act, self.w_down, ws.get(tag + "_out", T, self.hidden_size, self.dtype), T, allow_partial=FUSE_PARTIALS)
 
 

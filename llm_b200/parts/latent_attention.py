@@ -33,7 +33,7 @@ import torch
 
 from ..csrc import ops
 from .base import CacheNeed, ParamInfo, Part, build_part, register_part
-from .linear import FUSE_PARTIALS, linear
+from .linear import FUSE_PARTIALS, linear, linear_add
 
 _NAMES = {"q": "q", "down": "dkv", "down_norm": "dkv.norm", "up_k": "uk", "up_v": "uv", "gate": "g", "out": "o",
           "q_down": "dq", "q_down_norm": "dq.norm", "q_up": "uq", "sink": "sink"}
@@ -179,7 +179,7 @@ class LatentAttention(Part):
     def state_need(self):
         return None
 
-    def _forward_rotary(self, x: torch.Tensor, ctx, view) -> torch.Tensor:
+    def _forward_rotary(self, x: torch.Tensor, ctx, view, into=None):
         """The projections (float32 out, or split-K partial results: what is normed or turned next is not rounded before); norms,
         turning and the cache row; the per-head map of the queries to the cached row's layout; the paged attention with one
         key/value head (window, sink); the per-head value map; the output projection.  Without a query latent one product and
@@ -210,11 +210,13 @@ class LatentAttention(Part):
                             sink_values=self.sink_values)
         attn = ws.get("attn_out", T, H * self.value_dim, self.dtype)
         ops.gemm_heads(o_lat, self.w_uv, attn, T, H)
+        if into is not None and linear_add(attn, self.w_o, into.resid, T):
+            return None
         return linear(attn, self.w_o, ws.get("mixer_out", T, self.hidden_size, self.dtype), T, allow_partial=FUSE_PARTIALS)
 
-    def forward(self, x: torch.Tensor, ctx, view) -> torch.Tensor:
+    def forward(self, x: torch.Tensor, ctx, view, into=None):
         if self.rotary:
-            return self._forward_rotary(x, ctx, view)
+            return self._forward_rotary(x, ctx, view, into)
         T, ws = ctx.n_tokens, ctx.workspace
         H, R, RW = self.num_heads, self.rank, self.row_width
         proj = linear(x, self.w_in, ws.get("latent_in", T, self.w_in.shape[0], self.dtype), T)
@@ -230,6 +232,8 @@ class LatentAttention(Part):
         ops.paged_attention(o_lat, q_lat, pages, pages, view.group, ctx, H, 1, RW, 0, self.scale)
         attn = ws.get("attn_out", T, H * self.value_dim, self.dtype)
         ops.gemm_heads(o_lat, self.w_uv, attn, T, H, gate=gate)
+        if into is not None and linear_add(attn, self.w_o, into.resid, T):
+            return None
         return linear(attn, self.w_o, ws.get("mixer_out", T, self.hidden_size, self.dtype), T, allow_partial=FUSE_PARTIALS)
 
 

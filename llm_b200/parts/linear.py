@@ -33,7 +33,10 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, rows: int, 
         return out
     if bias is not None:
         allow_partial = False
-    if x.dtype == torch.bfloat16 and ops.gemm_fast_available(x, weight, out, rows):
+    if isinstance(x, ops.NormedRows):
+        sums = allow_partial and out.dtype != torch.float32
+        res = ops.gemm_few_sums(x, weight, rows, out.dtype) if sums else ops.gemm_few(x, weight, out, rows)
+    elif x.dtype == torch.bfloat16 and ops.gemm_fast_available(x, weight, out, rows):
         res = ops.gemm_fast(x, weight, out, rows, allow_partial=allow_partial, cta_limit=cta_limit)
     else:
         ops.gemm_simt(x, weight, out, rows)
@@ -43,6 +46,15 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, rows: int, 
     return res
 
 
+def linear_add(x: torch.Tensor, weight: torch.Tensor, resid: torch.Tensor, rows: int) -> bool:
+    """resid[:rows] += x[:rows] @ weight.T, float32, in the product's epilogue.  Returns False, having done nothing, where there are more rows
+    than the few-row product takes (or float32 operands): the caller then leaves the sum to the next norm."""
+    if rows == 0 or not ops.gemm_few_available(x, weight, rows):
+        return rows == 0
+    ops.gemm_few(x, weight, resid, rows, kind="add")
+    return True
+
+
 def linear_swiglu(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, rows: int, act: str = "silu") -> bool:
     """out[:rows] = act(x @ gate.T) * (x @ up.T) for weight = [gate; up] stacked along its rows and act silu or relu,
     with the activation applied in the product's epilogue.  Returns False, having done nothing,
@@ -50,6 +62,9 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, rows
     that the product splits its K dimension): the caller then runs the product and the activation
     kernel."""
     if rows == 0:
+        return True
+    if act in ("silu", "relu") and ops.gemm_few_available(x, weight, rows):
+        ops.gemm_few(x, weight, out, rows, kind=act)
         return True
     if x.dtype != torch.bfloat16 or not ops.gemm_swiglu_available(x, weight, out, rows):
         return False

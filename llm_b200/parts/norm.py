@@ -58,6 +58,14 @@ class RMSNorm(Part):
         stream.pending = None
         return out
 
+    def unformed(self, stream: ResidualStream):
+        """The stream's rows under this norm, for a product of few rows that norms what it reads (ops.NormedRows); None where the stream has
+        a term pending, or more rows than such a product takes."""
+        if (self.dtype != torch.bfloat16 or type(self).forward is not RMSNorm.forward or stream.pending is not None
+                or not ops.gemm_few_takes(stream.rows, self.size)):
+            return None
+        return ops.NormedRows(stream.resid, self.gain, self.eps, stream.rows, self.dtype)
+
     takes_unsummed = True      # attach() takes a sublayer's result before its last sums (what ops.add_rmsnorms takes)
 
     def attach(self, stream: ResidualStream, y, mult: float = 1.0) -> None:

@@ -1,0 +1,88 @@
+"""The products of a few rows (gemm_few.cu) at the edges of their tiles, boxes and rows, against float64 sums of the same bfloat16 operands."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from llm_b200.csrc import ops
+    return ops
+
+
+def operands(M, N, K, seed=0):
+    g = torch.Generator(device=DEV).manual_seed(seed + M * 7 + N * 3 + K)
+    a = torch.randn(M, K, generator=g, device=DEV).to(torch.bfloat16)
+    w = (torch.randn(N, K, generator=g, device=DEV) * 0.05).to(torch.bfloat16)
+    return a, w
+
+
+# K: one block, a box and a ragged one, several steps with a ragged last; N: fewer than SMs, no multiple of a tile, several tiles a CTA
+SIZES = [(96, 64), (17, 512), (2369, 576), (300, 1408), (2560, 2048), (5000, 2624)]
+# float32 sums of K terms in blocks: (K / 64 + 64) roundings of 2^-24 at most on the largest partial sum, as a share of the terms' norm
+BOUND = 2e-6
+
+
+@pytest.mark.parametrize("M", [1, 3, 7, 8])
+@pytest.mark.parametrize("N,K", SIZES)
+def test_sums(ops, M, N, K):
+    a, w = operands(M, N, K)
+    assert ops.gemm_few_available(a, w, M)
+    exact = a.double() @ w.double().T
+    scale = (a.double().abs() @ w.double().abs().T)
+    out = torch.full((M + 1, N + 3), 7.0, device=DEV)
+    ops.gemm_few(a, w, out[:, :N], M)
+    assert bool(((out[:M, :N].double() - exact).abs() <= BOUND * scale + 1e-30).all())
+    assert bool((out[M] == 7).all()) and bool((out[:, N:] == 7).all())            # nothing beside the results
+    half = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    ops.gemm_few(a, w, half, M)
+    assert torch.equal(half, out[:M, :N].to(torch.bfloat16))
+    resid = torch.randn(M, N, device=DEV)
+    added = resid.clone()
+    ops.gemm_few(a, w, added, M, kind="add")
+    assert torch.equal(added, resid + out[:M, :N])
+
+
+@pytest.mark.parametrize("M", [1, 5, 8])
+@pytest.mark.parametrize("N,K", [(34, 64), (2370, 576), (1408, 2048)])
+@pytest.mark.parametrize("act", ["silu", "relu"])
+def test_gated(ops, M, N, K, act):
+    a, w = operands(M, 2 * N, K)
+    z = a.double() @ w.double().T
+    scale = a.double().abs() @ w.double().abs().T
+    g, u = z[:, :N], z[:, N:]
+    ref = (torch.nn.functional.silu(g) if act == "silu" else torch.relu(g)) * u
+    out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    ops.gemm_few(a, w, out, M, kind=act)
+    # one rounding of the result, and the sums' errors through a product whose factors have slopes of at most 1.1
+    slack = 2.0 ** -8 * ref.abs() + 1.2 * BOUND * (scale[:, :N] * u.abs() + scale[:, N:] * g.abs()) + 1e-12
+    assert bool(((out.double() - ref).abs() <= slack).all())
+
+
+@pytest.mark.parametrize("M", [1, 2, 8])
+@pytest.mark.parametrize("N,K", [(40, 64), (300, 1408), (2560, 2048)])
+def test_rows_under_a_norm(ops, M, N, K):
+    _, w = operands(M, N, K)
+    x = torch.randn(M + 2, K, device=DEV) * torch.tensor([0.01, 300.0] * (M + 2), device=DEV)[:M + 2, None]
+    gain = 1.0 + 0.1 * torch.randn(K, device=DEV)
+    out = torch.empty(M, N, device=DEV)
+    ops.gemm_few(ops.NormedRows(x, gain, 1e-5, M, torch.bfloat16), w, out, M)
+    xd = x[:M].double()
+    h = xd / torch.sqrt((xd * xd).mean(-1, keepdim=True) + 1e-5) * gain.double()
+    # one rounding to bfloat16 (2^-9 of each) of what multiplies the weights, the rest in float32
+    scale = h.abs() @ w.double().abs().T
+    assert bool(((out.double() - h @ w.double().T).abs() <= (2.0 ** -9 + 1e-5) * scale).all())
+
+
+def test_what_is_not_taken(ops):
+    a, w = operands(8, 64, 128)
+    assert not ops.gemm_few_available(a.float(), w.float(), 8)
+    assert not ops.gemm_few_available(torch.cat([a, a]), w, 9)                    # more than eight rows
+    assert not ops.gemm_few_available(a[:, :96], w[:, :96], 8)                    # K off the 64-grid
+    assert not ops.gemm_few_available(a[:, 4:68], w[:, :64], 8)                   # rows off the 16-byte grid
+    assert not ops.gemm_few_takes(8, 16384)                                       # rows that leave no room for the stages
+    for rows in range(0, 18):
+        for k in (64, 96, 2048, 4096, 5632, 14336, 16384, 65536):
+            assert bool(ops.load_tensor().llmk_gemm_few_supported(rows, k)) == ops.gemm_few_takes(rows, k), (rows, k)
