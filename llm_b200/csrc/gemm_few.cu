@@ -25,28 +25,6 @@ constexpr int FEW_WARPS = 8;                      // that multiply; one more bri
 constexpr int FEW_BLOCK = 64;                     // k of a warp in a step
 constexpr int FEW_BOX = FEW_WARPS * FEW_BLOCK;
 constexpr int FEW_RED = 160;                      // floats of a warp's 16 x 8 accumulators in shared memory: 8 rows with a pitch of 20
-constexpr int FEW_MAX_STAGES = 16;
-
-enum : int { FEW_OUT_F32 = 0, FEW_OUT_BF16 = 1, FEW_OUT_ADD = 2, FEW_OUT_SILU = 3, FEW_OUT_RELU = 4 };
-
-struct FewArgs {
-  const __nv_bfloat16* a;      // rows, or
-  const float* x;              // rows of the residual stream with
-  const float* gain;           // the norm's gain and
-  float eps, inv_k;            // its epsilon; 1 / K
-  long long lda;               // of a or x
-  void* out;
-  long long ldo;
-  int M, N, K;                 // N: outputs (gated: half the weight rows)
-  int tile;                    // weight rows of a tile (gated: gate rows, as many up rows), up to 16 (8)
-  int tiles, stages, boxes;    // boxes: of a step
-  int* error;
-};
-
-// Shared memory: [stages][stage] [rows: (block, half, row, quad) of 16 bytes] [gain, under a norm] [sums] [squares] [barriers]
-inline int few_rest(int M, int K, bool normed) {
-  return K * M * 2 + (normed ? K * 4 : 0) + 2 * FEW_WARPS * FEW_RED * 4 + FEW_WARPS * 32 + (2 * FEW_MAX_STAGES + 1) * 8;
-}
 
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
   asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_addr(dst)),
@@ -79,9 +57,34 @@ __device__ __forceinline__ void sts16(uint32_t at, const uint4& v) {
 __device__ __forceinline__ void sts8(uint32_t at, uint32_t x, uint32_t y) { asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at), "r"(x), "r"(y) : "memory"); }
 __device__ __forceinline__ void sts(uint32_t at, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory"); }
 
-// OUT: what becomes of the sums.
-template <int OUT>
-__global__ void __launch_bounds__(FEW_WARPS * 32 + 32) few_rows_kernel(const __grid_constant__ CUtensorMap weights, const FewArgs p) {
+constexpr int FEW_MAX_STAGES = 16;
+
+enum : int { FEW_OUT_F32 = 0, FEW_OUT_BF16 = 1, FEW_OUT_ADD = 2, FEW_OUT_SILU = 3, FEW_OUT_RELU = 4 };
+
+struct FewArgs {
+  const __nv_bfloat16* a;      // rows, or
+  const float* x;              // rows of the residual stream with
+  const float* gain;           // the norm's gain and
+  float eps, inv_k;            // its epsilon; 1 / K
+  long long lda;               // of a or x
+  void* out;
+  long long ldo;
+  int M, N, K;                 // N: outputs (gated: half the weight rows)
+  int tile;                    // weight rows of a tile (gated: gate rows, as many up rows), up to 16 (8)
+  int tiles, stages, boxes;    // boxes: of a step
+  int* error;
+};
+
+// Shared memory: [stages][stage] [rows: (block, half, row, quad) of 16 bytes] [gain, under a norm] [sums] [squares] [barriers]
+inline int few_rest(int M, int K, bool normed) {
+  return K * M * 2 + (normed ? K * 4 : 0) + 2 * FEW_WARPS * FEW_RED * 4 + FEW_WARPS * 32 + (2 * FEW_MAX_STAGES + 1) * 8;
+}
+
+// OUT: what becomes of the sums.  KEEP: K of up to four boxes; a step is a tile then, and a lane keeps its part of the rows in registers over its
+// tiles (the products are bound by what they read from shared memory once the weights are there: 16 KB a box, and 8 more for the rows).
+template <int OUT, bool KEEP>
+__global__ void __launch_bounds__(FEW_WARPS * 32 + 32)
+few_rows_kernel(const __grid_constant__ CUtensorMap weights, const __grid_constant__ CUtensorMap weights_tail, const FewArgs p) {
   constexpr bool GATED = OUT == FEW_OUT_SILU || OUT == FEW_OUT_RELU;
   pdl_launch_dependents();
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -114,10 +117,12 @@ __global__ void __launch_bounds__(FEW_WARPS * 32 + 32) few_rows_kernel(const __g
         ok = tc::mbar_wait(empty + s, phase);
         if (!ok) break;
         const int end = min(b + p.boxes, all_boxes);
-        tc::mbar_arrive_expect_tx(full + s, (end - b) * box_bytes);
+        const int missing = max(0, end * FEW_WARPS - blocks);      // a ragged last box has a map of its own: none reaches past K
+        tc::mbar_arrive_expect_tx(full + s, (end - b) * box_bytes - missing * (box_bytes / FEW_WARPS));
         for (unsigned char* dst = smem + s * stage_bytes; b < end; ++b, dst += box_bytes) {
-          tma_load_3d(dst, &weights, 0, n, b * FEW_WARPS, full + s);
-          if (GATED) tma_load_3d(dst + half_box, &weights, 0, p.N + n, b * FEW_WARPS, full + s);
+          const CUtensorMap* map = (b + 1) * FEW_WARPS <= blocks ? &weights : &weights_tail;
+          tma_load_3d(dst, map, 0, n, b * FEW_WARPS, full + s);
+          if (GATED) tma_load_3d(dst + half_box, map, 0, p.N + n, b * FEW_WARPS, full + s);
         }
         ++issued;
         if (++s == p.stages) { s = 0; phase ^= 1; }
@@ -214,23 +219,30 @@ __global__ void __launch_bounds__(FEW_WARPS * 32 + 32) few_rows_kernel(const __g
   }
   const uint32_t act_at = acts + (warp * 2 * p.M + min(row, p.M - 1)) * 64 + quad * 16;
   const int act_box = FEW_WARPS * 2 * p.M * 64, act_half = p.M * 64;
-  struct Operands { uint4 lo[2], hi[2], b[2]; };
-  auto load = [&](Operands& o, int weight, int act) {
+  struct Weights { uint4 lo[2], hi[2]; };
+  struct Rows { uint4 b[2]; };
+  auto load = [&](Weights& o, int weight) {
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      o.lo[j] = lds16(lo_at[j] + weight);
-      o.hi[j] = lds16(hi_at[j] + weight);
-      o.b[j] = lds16(act_at + act + j * act_half);
-    }
+    for (int j = 0; j < 2; ++j) { o.lo[j] = lds16(lo_at[j] + weight); o.hi[j] = lds16(hi_at[j] + weight); }
   };
-  auto multiply = [&](float (&c)[2][4], const Operands& o) {
+  auto load_rows = [&](Rows& o, int box) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) o.b[j] = lds16(act_at + box * act_box + j * act_half);
+  };
+  auto multiply = [&](float (&c)[2][4], const Weights& o, const Rows& r) {
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       const uint32_t a0[4] = {o.lo[j].x, o.hi[j].x, o.lo[j].y, o.hi[j].y}, a1[4] = {o.lo[j].z, o.hi[j].z, o.lo[j].w, o.hi[j].w};
-      mma(c[0], a0, o.b[j].x, o.b[j].y);
-      mma(c[1], a1, o.b[j].z, o.b[j].w);
+      mma(c[0], a0, r.b[j].x, r.b[j].y);
+      mma(c[1], a1, r.b[j].z, r.b[j].w);
     }
   };
+  Rows kept[4];
+  if (KEEP) {
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+      if (b * FEW_WARPS + warp < blocks) load_rows(kept[b], b);
+  }
   const int out_row = threadIdx.x & 15, out_token = threadIdx.x >> 4;
   int s = 0, buffer = 0;
   uint32_t phase = 0;
@@ -242,24 +254,43 @@ __global__ void __launch_bounds__(FEW_WARPS * 32 + 32) few_rows_kernel(const __g
     float before = 0.f;
     if (OUT == FEW_OUT_ADD && mine) before = reinterpret_cast<float*>(p.out)[(size_t)out_token * p.ldo + n];
     float c[2][4] = {};
-#pragma unroll 1
-    for (int b = 0; b < all_boxes;) {
-      ok = ok && tc::mbar_wait(full + s, phase);
-      const int end = min(b + p.boxes, all_boxes);
-      int weight = s * stage_bytes;
-#pragma unroll 1
-      for (; b < end; b += 2, weight += 2 * box_bytes) {      // a pair of boxes: all of their loads, then the products
-        Operands one, two;
-        const bool first = b * FEW_WARPS + warp < blocks, second = b + 1 < end && (b + 1) * FEW_WARPS + warp < blocks;
-        if (first) load(one, weight, b * act_box);
-        if (second) load(two, weight + box_bytes, (b + 1) * act_box);
-        if (first) multiply(c, one);
-        if (second) multiply(c, two);
-      }
-      b = end;
+    auto release = [&]() {
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(empty + s);
       if (++s == p.stages) { s = 0; phase ^= 1; }
+    };
+    if (KEEP) {
+      ok = ok && tc::mbar_wait(full + s, phase);
+      const int weight = s * stage_bytes;
+#pragma unroll
+      for (int b = 0; b < 4; b += 2) {                          // a pair of boxes: all of their loads, then the products
+        Weights one, two;
+        const bool first = b * FEW_WARPS + warp < blocks, second = (b + 1) * FEW_WARPS + warp < blocks;
+        if (first) load(one, weight + b * box_bytes);
+        if (second) load(two, weight + (b + 1) * box_bytes);
+        if (first) multiply(c, one, kept[b]);
+        if (second) multiply(c, two, kept[b + 1]);
+      }
+      release();
+    } else {
+#pragma unroll 1
+      for (int b = 0; b < all_boxes;) {
+        ok = ok && tc::mbar_wait(full + s, phase);
+        const int end = min(b + p.boxes, all_boxes);
+        int weight = s * stage_bytes;
+#pragma unroll 1
+        for (; b < end; b += 2, weight += 2 * box_bytes) {
+          Weights one, two;
+          Rows x, y;
+          const bool first = b * FEW_WARPS + warp < blocks, second = b + 1 < end && (b + 1) * FEW_WARPS + warp < blocks;
+          if (first) { load(one, weight); load_rows(x, b); }
+          if (second) { load(two, weight + box_bytes); load_rows(y, b + 1); }
+          if (first) multiply(c, one, x);
+          if (second) multiply(c, two, y);
+        }
+        b = end;
+        release();
+      }
     }
     const uint32_t put = red + ((buffer * FEW_WARPS + warp) * FEW_RED + 2 * quad * 20 + row) * 4;
     sts(put, c[0][0] + c[1][0]);
@@ -308,26 +339,28 @@ EncodeFewFn encode_few_fn() {
   return fn;
 }
 
-// w [rows, K] as [K / 64][rows][64]: a box is `tile` rows of eight blocks of 64 k, each a 128-byte line.
-int encode_weights(CUtensorMap* out, const void* w, int rows, int K, long long ldw, int tile) {
+// w [rows, K] as [K / 64][rows][64]; a box holds `blocks` blocks of `tile` rows.
+int encode_weights(CUtensorMap* out, const void* w, long long rows, int K, long long ldw, int tile, int blocks) {
   EncodeFewFn fn = encode_few_fn();
   if (!fn) return llmk_fail(-2, "cuTensorMapEncodeTiled is not available from the driver");
   cuuint64_t dims[3] = {(cuuint64_t)FEW_BLOCK, (cuuint64_t)rows, (cuuint64_t)(K / FEW_BLOCK)}, strides[2] = {(cuuint64_t)ldw * 2, FEW_BLOCK * 2};
-  cuuint32_t box[3] = {FEW_BLOCK, (cuuint32_t)tile, FEW_WARPS}, step[3] = {1, 1, 1};
+  cuuint32_t box[3] = {FEW_BLOCK, (cuuint32_t)tile, (cuuint32_t)blocks}, step[3] = {1, 1, 1};
   CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(w), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : llmk_fail(-2, "cuTensorMapEncodeTiled failed with %d", (int)r);
 }
 
-int launch_few(const CUtensorMap& map, const FewArgs& p, int out_kind, int grid, size_t smem, cudaStream_t stream) {
-  void (*kern)(CUtensorMap, FewArgs) = out_kind == FEW_OUT_F32 ? few_rows_kernel<FEW_OUT_F32> : out_kind == FEW_OUT_BF16 ? few_rows_kernel<FEW_OUT_BF16>
-                                       : out_kind == FEW_OUT_ADD ? few_rows_kernel<FEW_OUT_ADD> : out_kind == FEW_OUT_SILU ? few_rows_kernel<FEW_OUT_SILU>
-                                       : few_rows_kernel<FEW_OUT_RELU>;
+template <bool KEEP>
+int launch_few(const CUtensorMap& map, const CUtensorMap& tail, const FewArgs& p, int out_kind, int grid, size_t smem, cudaStream_t stream) {
+  void (*kern)(CUtensorMap, CUtensorMap, FewArgs) =
+      out_kind == FEW_OUT_F32 ? few_rows_kernel<FEW_OUT_F32, KEEP> : out_kind == FEW_OUT_BF16 ? few_rows_kernel<FEW_OUT_BF16, KEEP>
+      : out_kind == FEW_OUT_ADD ? few_rows_kernel<FEW_OUT_ADD, KEEP> : out_kind == FEW_OUT_SILU ? few_rows_kernel<FEW_OUT_SILU, KEEP>
+      : few_rows_kernel<FEW_OUT_RELU, KEEP>;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return llmk_fail((int)e, "gemm_few: %s", cudaGetErrorString(e));
   }
-  launch_kernel(kern, dim3(grid), dim3(FEW_WARPS * 32 + 32), smem, stream, map, p);
+  launch_kernel(kern, dim3(grid), dim3(FEW_WARPS * 32 + 32), smem, stream, map, tail, p);
   LLMK_LAUNCH_CHECK("gemm_few");
 }
 
@@ -364,18 +397,23 @@ LLMK_API int llmk_gemm_few(const void* a, const float* x, const float* gain, flo
   const int grid = p.tiles < sms ? p.tiles : sms;
   const int box_bytes = (gated ? 2 : 1) * p.tile * 1024, all_boxes = (K + FEW_BOX - 1) / FEW_BOX;
   const int rest = few_rest(M, K, x != nullptr), room = FEW_SMEM - rest < FEW_RING ? FEW_SMEM - rest : FEW_RING;
+  const bool keep = all_boxes <= 4 && room >= 2 * all_boxes * box_bytes;
   // four boxes a step (a step costs a wait) while three steps fit, or all there are; else two, else one
   for (p.boxes = 4;; p.boxes /= 2) {
     if (p.boxes > all_boxes) p.boxes = all_boxes;
     const int all = ((p.tiles + sms - 1) / sms) * ((all_boxes + p.boxes - 1) / p.boxes), fit = room / (p.boxes * box_bytes);
     p.stages = all < fit ? all : fit;
-    if (p.boxes == 1 || p.stages >= 3 || p.stages >= all) break;
+    if (keep || p.boxes == 1 || p.stages >= 3 || p.stages >= all) break;
   }
   if (p.stages > FEW_MAX_STAGES) p.stages = FEW_MAX_STAGES;
   // at least half of the shared memory: a CTA that shared its SM with another of the same launch would end long after the rest (a kernel that
   // starts while the one before it leaves SMs finds room for two on some: a decode step of 1.1 B then took 880 us instead of 720)
   const size_t need = rest + (size_t)p.stages * p.boxes * box_bytes, smem = need < FEW_SMEM / 2 + 1024 ? FEW_SMEM / 2 + 1024 : need;
-  CUtensorMap map;
-  if (int rc = encode_weights(&map, w, gated ? 2 * N : N, K, ldw, p.tile)) return rc;
-  return launch_few(map, p, out_kind, grid, smem, stream);
+  CUtensorMap map, tail;
+  const int last = K / FEW_BLOCK % FEW_WARPS, w_rows = gated ? 2 * N : N;
+  if (int rc = encode_weights(&map, w, w_rows, K, ldw, p.tile, all_boxes == 1 && last ? last : FEW_WARPS)) return rc;
+  tail = map;
+  if (last)
+    if (int rc = encode_weights(&tail, w, w_rows, K, ldw, p.tile, last)) return rc;
+  return keep ? launch_few<true>(map, tail, p, out_kind, grid, smem, stream) : launch_few<false>(map, tail, p, out_kind, grid, smem, stream);
 }

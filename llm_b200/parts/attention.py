@@ -195,11 +195,12 @@ class PagedAttention(Part):
     def reads_unformed(self, rows, ctx) -> bool:
         return not self.extended and ops.gemm_few_available(rows, self.w_qkv, ctx.n_tokens)
 
-    def forward(self, x: torch.Tensor, ctx, view, into=None):
+    def forward(self, x: torch.Tensor, ctx, view, into=None, whole: bool = False):
+        """into: the stream that a last product of few rows may add to (the result is then None); whole: no unsummed result."""
         T = ctx.n_tokens
         ws = ctx.workspace
         if self.extended:
-            return self._forward_extended(x, ctx, view, into)
+            return self._forward_extended(x, ctx, view, into, whole)
         width = self.q_size + 2 * self.kv_size
         cos = sin = None
         own_transform = None
@@ -229,7 +230,8 @@ class PagedAttention(Part):
             if q is not None:
                 ops.paged_attention(attn, q, k_pages, v_pages, view.group, ctx, self.num_heads, k_pages.shape[1],
                                     self.head_dim, self.window or 0, self.scale)
-                return linear(attn, self.w_o, ws.get("mixer_out", T, self.hidden_size, self.dtype), T, allow_partial=FUSE_PARTIALS)
+                return linear(attn, self.w_o, ws.get("mixer_out", T, self.hidden_size, self.dtype), T,
+                              allow_partial=FUSE_PARTIALS and not whole)
             qkv = linear(x, self.w_qkv, ws.get("qkv", T, width, self.dtype), T, allow_partial=FUSE_PARTIALS,
                          cta_limit=self._qkv_cta_limit(ctx, k_pages))
         ops.rope_store_attend(attn, qkv, cos, sin, k_pages, v_pages, view.group, ctx, self.num_heads,
@@ -238,11 +240,11 @@ class PagedAttention(Part):
                               q_rot=lambda: ws.get("q_rot", T, self.q_size, self.dtype))
         if into is not None and self.b_o is None and linear_add(attn, self.w_o, into.resid, T):
             return None
-        return linear(attn, self.w_o, ws.get("mixer_out", T, self.hidden_size, self.dtype), T, allow_partial=FUSE_PARTIALS,
-                      bias=self.b_o)
+        return linear(attn, self.w_o, ws.get("mixer_out", T, self.hidden_size, self.dtype), T,
+                      allow_partial=FUSE_PARTIALS and not whole, bias=self.b_o)
 
 
-    def _forward_extended(self, x: torch.Tensor, ctx, view, into=None):
+    def _forward_extended(self, x: torch.Tensor, ctx, view, into=None, whole: bool = False):
         """One product for q, k, v (its split-K partial results go unsummed to the next kernel); one kernel that
         sums them, turns the pairs of q and k and stores k and v in the pages; the attention kernel that takes
         the options; the output projection."""
@@ -274,7 +276,7 @@ class PagedAttention(Part):
                             dist_bias=(self.r1, self.r2) if self.dist_bias else None)
         if into is not None and linear_add(attn, self.w_o, into.resid, T):
             return None
-        return linear(attn, self.w_o, ws.get("mixer_out", T, self.hidden_size, self.dtype), T, allow_partial=FUSE_PARTIALS)
+        return linear(attn, self.w_o, ws.get("mixer_out", T, self.hidden_size, self.dtype), T, allow_partial=FUSE_PARTIALS and not whole)
 
 
 register_part("mixer", "attention", PagedAttention)

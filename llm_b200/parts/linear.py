@@ -33,7 +33,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, rows: int, 
         return out
     if bias is not None:
         allow_partial = False
-    if isinstance(x, ops.NormedRows):
+    if ops.gemm_few_available(x, weight, rows):
         sums = allow_partial and out.dtype != torch.float32
         res = ops.gemm_few_sums(x, weight, rows, out.dtype) if sums else ops.gemm_few(x, weight, out, rows)
     elif x.dtype == torch.bfloat16 and ops.gemm_fast_available(x, weight, out, rows):

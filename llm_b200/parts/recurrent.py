@@ -21,6 +21,7 @@ step sizes, states and the norms are float32; projections and convolutions run i
 from __future__ import annotations
 
 import dataclasses
+import inspect
 
 import torch
 
@@ -479,6 +480,7 @@ class ParallelMixers(Part):
         self.hidden_size, self.eps = int(hidden_size), float(eps)
         self.left_name, self.right_name = left_name, right_name
         self.left, self.right = build_part("mixer", left, dtype, device), build_part("mixer", right, dtype, device)
+        self.left_whole = "whole" in inspect.signature(self.left.forward).parameters
         if self.left.cache_need() is not None and self.right.cache_need() is not None:
             raise ValueError("parallel mixers: only one side may keep keys and values")
         self.left_cols = _pad4(_state_numel(self.left.state_need()))
@@ -517,8 +519,10 @@ class ParallelMixers(Part):
         T, ws = ctx.n_tokens, ctx.workspace
         ls = view.state[:, :self.left_cols] if self.left_cols else None
         rs = view.state[:, self.left_cols:] if self.right_cols else None
-        a = self.left.forward(x, ctx, _sub_view(view, ls))
-        # unsummed partial results live until the next product: the left side's are summed before the right side runs
+        # unsummed partial results live until the next product: the left side's are summed before the right side runs (by its last
+        # product itself where that has few rows)
+        whole = {"whole": True} if self.left_whole and T <= ops.FEW_ROWS else {}
+        a = self.left.forward(x, ctx, _sub_view(view, ls), **whole)
         a = ops.settle(a, ws.get("parallel_left", T, self.hidden_size, self.dtype), T)
         b = self.right.forward(x, ctx, _sub_view(view, rs))
         if allow_unsummed and self.leaves_unsummed:
