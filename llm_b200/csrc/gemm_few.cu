@@ -72,12 +72,13 @@ struct FewArgs {
   int M, N, K;                 // N: outputs (gated: half the weight rows)
   int tile;                    // weight rows of a tile (gated: gate rows, as many up rows), up to 16 (8)
   int tiles, stages, boxes;    // boxes: of a step
+  int early;                   // steps that are asked for before the rows
   int* error;
 };
 
 // Shared memory: [stages][stage] [rows: (block, half, row, quad) of 16 bytes] [gain, under a norm] [sums] [squares] [barriers]
 inline int few_rest(int M, int K, bool normed) {
-  return K * M * 2 + (normed ? K * 4 : 0) + 2 * FEW_WARPS * FEW_RED * 4 + FEW_WARPS * 32 + (2 * FEW_MAX_STAGES + 1) * 8;
+  return K * M * 2 + (normed ? K * 4 : 0) + 2 * FEW_WARPS * FEW_RED * 4 + FEW_WARPS * 32 + (2 * FEW_MAX_STAGES + 2) * 8;
 }
 
 // OUT: what becomes of the sums.  KEEP: K of up to four boxes; a step is a tile then, and a lane keeps its part of the rows in registers over its
@@ -96,10 +97,12 @@ few_rows_kernel(const __grid_constant__ CUtensorMap weights, const __grid_consta
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + (squares + FEW_WARPS * 8 * 4 - ring));         // [stages]
   uint64_t* empty = full + p.stages;                                                         // [stages]
   uint64_t* gain_bar = empty + p.stages;
+  uint64_t* asked = gain_bar + 1;                  // the rows are on their way
   if (threadIdx.x == 0) {
     tc::prefetch_tensormap(&weights);
     for (int s = 0; s < p.stages; ++s) { tc::mbar_init(full + s, 1); tc::mbar_init(empty + s, FEW_WARPS); }
     tc::mbar_init(gain_bar, 1);
+    tc::mbar_init(asked, FEW_WARPS);
     tc::fence_mbar_init();
   }
   __syncthreads();
@@ -114,7 +117,9 @@ few_rows_kernel(const __grid_constant__ CUtensorMap weights, const __grid_consta
     for (int tile = blockIdx.x; ok && tile < p.tiles; tile += gridDim.x) {
       const int n = min(tile * p.tile, p.N - p.tile);  // the last tile ends with the weights, and repeats rows of the one before
       for (int b = 0; b < all_boxes;) {
-        ok = tc::mbar_wait(empty + s, phase);
+        // what a load waits for is what was asked for before it: the rows come before all but the first steps
+        if (issued == p.early) ok = tc::mbar_wait(asked, 0);
+        ok = ok && tc::mbar_wait(empty + s, phase);
         if (!ok) break;
         const int end = min(b + p.boxes, all_boxes);
         const int missing = max(0, end * FEW_WARPS - blocks);      // a ragged last box has a map of its own: none reaches past K
@@ -136,6 +141,7 @@ few_rows_kernel(const __grid_constant__ CUtensorMap weights, const __grid_consta
   }
 
   pdl_wait();
+  if (warp >= blocks && lane == 0) tc::mbar_arrive(asked);      // none of its own
   // the rows, the warp's blocks warp, warp + 8, ...: [block][half of a lane's 16 k][row][quad] of 16 bytes, all lanes along k
   bool ok = true;
   if (p.x) {
@@ -157,6 +163,7 @@ few_rows_kernel(const __grid_constant__ CUtensorMap weights, const __grid_consta
           if (r < p.M && block[i] < blocks)
             v[r][i] = *reinterpret_cast<const float4*>(p.x + (size_t)r * p.lda + block[i] * FEW_BLOCK + (lane & 15) * 4);
         }
+      if (b0 == warp && lane == 0) tc::mbar_arrive(asked);
       float q[8];
 #pragma unroll
       for (int r = 0; r < 8; ++r) {
@@ -199,6 +206,7 @@ few_rows_kernel(const __grid_constant__ CUtensorMap weights, const __grid_consta
 #pragma unroll
         for (int i = 0; i < 2; ++i)
           if (r < p.M && block[i] < blocks) v[r][i] = *reinterpret_cast<const uint4*>(p.a + (size_t)r * p.lda + block[i] * FEW_BLOCK + (lane & 7) * 8);
+      if (b0 == warp && lane == 0) tc::mbar_arrive(asked);
 #pragma unroll
       for (int r = 0; r < 8; ++r)
 #pragma unroll
@@ -365,9 +373,10 @@ int launch_few(const CUtensorMap& map, const CUtensorMap& tail, const FewArgs& p
 }
 
 constexpr int FEW_SMEM = 227 * 1024, FEW_LEAST_STAGES = 3;
-// The most that is in flight: what the rows' loads wait behind.  Decode steps of 1.1 B (1, 4, 8 rows) with 64, 100, 140, 200 KB: 771, 695, 666, 677;
-// 795, 712, 690, 719; 828, 746, 750, 755 us.
-constexpr int FEW_RING = 140 * 1000;
+// The most that is in flight, and how much of it is asked for before the rows, which wait behind that.  Decode steps of 1.1 B (1, 4, 8 rows), all of the
+// ring first: 64 KB 771, 795, 828 us; 100 KB 695, 712, 746; 140 KB 666, 690, 750; 200 KB 677, 719, 755 (649, 675, 738 with 140 KB once the rows
+// were kept in registers); of 140 KB first 96 KB: 634, 665, 717; 72 KB: 629, 667, 716; 57 KB: 638, 668, 727.
+constexpr int FEW_RING = 140 * 1000, FEW_EARLY = 72 * 1000;
 
 }  // namespace
 
@@ -406,6 +415,8 @@ LLMK_API int llmk_gemm_few(const void* a, const float* x, const float* gain, flo
     if (keep || p.boxes == 1 || p.stages >= 3 || p.stages >= all) break;
   }
   if (p.stages > FEW_MAX_STAGES) p.stages = FEW_MAX_STAGES;
+  p.early = FEW_EARLY / (p.boxes * box_bytes);
+  if (p.early < 1) p.early = 1;
   // at least half of the shared memory: a CTA that shared its SM with another of the same launch would end long after the rest (a kernel that
   // starts while the one before it leaves SMs finds room for two on some: a decode step of 1.1 B then took 880 us instead of 720)
   const size_t need = rest + (size_t)p.stages * p.boxes * box_bytes, smem = need < FEW_SMEM / 2 + 1024 ? FEW_SMEM / 2 + 1024 : need;

@@ -1996,7 +1996,7 @@ _FEW_KINDS = {"add": 2, "silu": 3, "relu": 4}
 @functools.lru_cache(maxsize=4096)
 def gemm_few_takes(rows: int, k: int) -> bool:
     """Whether the few-row product takes so many rows of k channels (as llmk_gemm_few_supported)."""
-    rest = k * rows * 2 + 4 * k + 2 * 8 * 160 * 4 + 256 + 33 * 8
+    rest = k * rows * 2 + 4 * k + 2 * 8 * 160 * 4 + 256 + 34 * 8
     return 0 < rows <= FEW_ROWS and k > 0 and k % 64 == 0 and rest + 3 * 16384 <= _FEW_SMEM
 
 
