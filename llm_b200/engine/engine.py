@@ -19,7 +19,7 @@ import ctypes
 import numpy as np
 import torch
 
-from ..cache.manager import CacheError, CacheManager, GroupSpec, OutOfPages
+from ..cache.manager import CacheError, CacheManager, GroupSpec, OutOfPages, address
 from ..cache.storage import CacheStorage, StateStorage, bytes_per_page
 from ..config.engine_options import EngineOptions
 from ..config.model_config import load_config, parse_config
@@ -357,9 +357,9 @@ class Engine:
         # the native routine writes tokens, positions, block tables, slot maps, wanted rows and the
         # rest of the step's metadata into the pinned block, from the pool's own tables
         lib, pool = cache.native
-        ptr = lambda a: a.ctypes.data_as(ctypes.c_void_p)
         n_feed = lib.llmh_prepare_step(pool, ctypes.byref(native_layout), ctypes.c_void_p(host_t.data_ptr()), B,
-                                       ptr(slots), ptr(ns), ptr(starts), ptr(tokens), ptr(want_counts), ptr(wants), ptr(feeds))
+                                       address(slots), address(ns), address(starts), address(tokens), address(want_counts),
+                                       address(wants), address(feeds))
         if n_feed < 0:
             raise StepError(lib.llmh_pool_error(pool).decode("utf-8", "replace"))
         entry_tokens, entry_start, entry_slots = ns, starts, slots
@@ -375,9 +375,9 @@ class Engine:
         a, b = lay.base, lay.used_end(B)
         self.meta[a:b].copy_(host_t[a:b], non_blocking=True)
         self.last_h2d_bytes = 4 * (b - a)
-        ev = torch.cuda.Event()
-        ev.record()
-        self._host_events[self._ring_at] = ev
+        if self._host_events[self._ring_at] is None:
+            self._host_events[self._ring_at] = torch.cuda.Event()
+        self._host_events[self._ring_at].record(ops.current_stream())      # _next_host_buffer has waited for what it recorded before
         if n_feed:
             ops.feed_tokens(ctx.token_ids, feed_source, self.meta[lay.feed_dst: lay.feed_dst + n_feed],
                             self.meta[lay.feed_src: lay.feed_src + n_feed], n_feed)
@@ -395,7 +395,7 @@ class Engine:
         return self._host_ring[self._ring_at]
 
     def _forward(self, ctx: StepContext) -> None:
-        ops.set_stream(torch.cuda.current_stream().cuda_stream)     # looked up once per step, not per kernel
+        ops.set_stream(ops.current_stream_handle())     # looked up once per step, not per kernel
         if self.dtype == torch.bfloat16:
             ops.set_error_block(self.status)
         try:

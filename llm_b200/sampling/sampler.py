@@ -90,7 +90,7 @@ class Sampler:
             ops.sample_rows(out, logits, rows)
         self._out_host[k].copy_(out, non_blocking=True)
         event = torch.cuda.Event()
-        event.record()
+        event.record(ops.current_stream())
         return SampleHandle(out, self._out_host[k], rows, event)
 
     def sample(self, logits: torch.Tensor, temperatures: Sequence[float], uniforms: Sequence[float]) -> List[int]:
