@@ -446,18 +446,26 @@ __device__ __forceinline__ void store_row32(TOut* row, const float (&v)[32], int
   }
 }
 
+// Maps of the weights for every width of tile, of which a grouped product takes one when it knows how many row tiles are in use (count 0: the
+// width it was launched with).  The host only knows the most there can be; with 24 row tiles of 16 experts, 2,048 channels in, a width of 256
+// takes 1,408 outputs in one round of 148 SMs instead of two of 128 (33.2 -> 30.2 us), 192 takes 2,048 outputs in two rounds
+// instead of two of 256 (33.9 -> 31.5 us).
+struct WidthMaps {
+  static constexpr int MOST = 5;
+  CUtensorMap map[MOST];
+  int width[MOST];
+  int count;
+};
+
 template <typename TOut, bool SWIGLU>
 __global__ void __launch_bounds__(THREADS, 1)
-gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q,
+gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q, const __grid_constant__ WidthMaps widths,
                           TOut* __restrict__ C, long long ldc, int M, int N, int K, int tile_q,
                           int* __restrict__ err_flag, const Grouping grp) {
   constexpr int BNQ = 256;
   constexpr int STAGES = stages_for(BNQ);
   constexpr int Q_STAGE_BYTES = q_stage_bytes(BNQ);
   constexpr uint32_t TMEM_COLS = 512;
-  const uint32_t IDESC = idesc_bf16_f32(BP, tile_q);
-  const uint32_t stage_tx = (uint32_t)(P_STAGE_BYTES + tile_q * BK * 2);
-
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* smem_p = smem;
@@ -471,7 +479,6 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_p, const __gri
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int inter = N / 2;                                 // SWIGLU: gate rows, and output columns
   int m_tiles = (M + BP - 1) / BP;
-  const int n_tiles = SWIGLU ? (inter + 127) / 128 : (N + tile_q - 1) / tile_q;
   const int nkb = (K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
@@ -500,6 +507,16 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_p, const __gri
     pdl_wait();
     m_tiles = min(m_tiles, *grp.n_tiles);
   }
+  // a tile takes as long as its loads, 128 + width rows a block of k: the width with the least of that over the rounds, where it is 5 % less
+  const CUtensorMap* weights = &map_q;
+  auto cost_of = [&](int w) { return (m_tiles * ((N + w - 1) / w) + (int)gridDim.x - 1) / (int)gridDim.x * (128 + w); };
+  for (int i = 0, best = cost_of(tile_q); i < widths.count; ++i) {
+    const int cost = cost_of(widths.width[i]);
+    if (cost * 20 < best * 19) { best = cost; tile_q = widths.width[i]; weights = &widths.map[i]; }
+  }
+  const uint32_t IDESC = idesc_bf16_f32(BP, tile_q);
+  const uint32_t stage_tx = (uint32_t)(P_STAGE_BYTES + tile_q * BK * 2);
+  const int n_tiles = SWIGLU ? (inter + 127) / 128 : (N + tile_q - 1) / tile_q;
   const int total_tiles = m_tiles * n_tiles;
   if (warp == 0) {
     if (lane == 0) {
@@ -516,9 +533,9 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_p, const __gri
           ok = mbar_wait(&empty_bar[s], ((it / STAGES) & 1) ^ 1);
           if (!ok) break;
           mbar_arrive_expect_tx(&full_bar[s], stage_tx);
-          tma_load_2d(smem_q + s * Q_STAGE_BYTES, &map_q, kb * BK, q0, &full_bar[s]);
+          tma_load_2d(smem_q + s * Q_STAGE_BYTES, weights, kb * BK, q0, &full_bar[s]);
           // the up rows of these gate rows: rows 128.. of the stage (a box is 128 rows of 128 bytes)
-          if (SWIGLU) tma_load_2d(smem_q + s * Q_STAGE_BYTES + 128 * 128, &map_q, kb * BK, inter + q0, &full_bar[s]);
+          if (SWIGLU) tma_load_2d(smem_q + s * Q_STAGE_BYTES + 128 * 128, weights, kb * BK, inter + q0, &full_bar[s]);
           tma_load_2d(smem_p + s * P_STAGE_BYTES, &map_p, kb * BK, p0, &full_bar[s]);
         }
       }
@@ -992,7 +1009,8 @@ int launch_cfg(const CUtensorMap& mp, const CUtensorMap& mq, void* C, long long 
 
 template <typename TOut, bool SWIGLU>
 int launch_persistent(const CUtensorMap& mp, const CUtensorMap& mq, void* C, long long ldc, int M, int N, int K,
-                      int tile_q, cudaStream_t stream, const Grouping grp = Grouping{0, 0, 0, nullptr, nullptr, -1, nullptr, 0}) {
+                      int tile_q, cudaStream_t stream, const Grouping grp = Grouping{0, 0, 0, nullptr, nullptr, -1, nullptr, 0},
+                      const WidthMaps& widths = WidthMaps{}) {
   auto kern = gemm_tc_persistent_kernel<TOut, SWIGLU>;
   constexpr int smem = smem_bytes_for(256);
   static bool configured = false;
@@ -1002,7 +1020,7 @@ int launch_persistent(const CUtensorMap& mp, const CUtensorMap& mq, void* C, lon
     configured = true;
   }
   const int tiles = ((M + BP - 1) / BP) * (SWIGLU ? (N / 2 + 127) / 128 : (N + tile_q - 1) / tile_q);
-  launch_kernel(kern, dim3(tiles < llmk_sm_count() ? tiles : llmk_sm_count()), dim3(THREADS), (size_t)smem, stream, mp, mq, (TOut*)C, ldc, M, N, K,
+  launch_kernel(kern, dim3(tiles < llmk_sm_count() ? tiles : llmk_sm_count()), dim3(THREADS), (size_t)smem, stream, mp, mq, widths, (TOut*)C, ldc, M, N, K,
                 tile_q, g_err_flag, grp);
   LLMK_LAUNCH_CHECK("gemm_tc_persistent");
 }
@@ -1236,8 +1254,13 @@ LLMK_API int llmk_gemm_tc_grouped(const void* A, const void* W, void* C, int M, 
   if (persistent && mode == 2 && (long long)(M / BP) * ((N + tile - 1) / tile) > llmk_sm_count()) {
     // more tiles than SMs (a prompt's experts): persistent CTAs with two accumulators, so that a tile's
     // epilogue runs under the next tile's products and no partial wave is left at the end
-    if (out_dtype == LLMK_F32) return launch_persistent<float, false>(mp, mq, C, ldc, M, N, K, tile, stream, grp);
-    if (out_dtype == LLMK_BF16) return launch_persistent<__nv_bfloat16, false>(mp, mq, C, ldc, M, N, K, tile, stream, grp);
+    WidthMaps widths{};
+    for (int w = 256; N >= 256 && w >= 128; w -= 32) {
+      if ((rc = get_map(&widths.map[widths.count], W, (uint64_t)groups * N, K, ldw, w))) return rc;
+      widths.width[widths.count++] = w;
+    }
+    if (out_dtype == LLMK_F32) return launch_persistent<float, false>(mp, mq, C, ldc, M, N, K, tile, stream, grp, widths);
+    if (out_dtype == LLMK_BF16) return launch_persistent<__nv_bfloat16, false>(mp, mq, C, ldc, M, N, K, tile, stream, grp, widths);
     return llmk_fail(-1, "gemm_tc_grouped: unsupported output kind %d", out_dtype);
   }
   const int splits = mode == 1 ? groups : 1;            // the grid's z: one product each
