@@ -100,6 +100,47 @@ inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// The same in thread-block clusters of `cluster` CTAs along x.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_clusters(void (*kernel)(KArgs...), dim3 grid, dim3 block, int cluster, cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cluster;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = llmk_pdl_enabled() ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+// All threads of a cluster of CTAS CTAs get the sum of `v`, in a fixed order: a CTA's by block_sum, the CTAs' by rank.  Every CTA hands its sum
+// to the others through distributed shared memory, once a launch, when all of them have called cluster_begin (at their start, all threads):
+// before that a neighbour's shared memory is not there to be written.
+__device__ __forceinline__ void cluster_begin() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+template <int CTAS>
+__device__ __forceinline__ float cluster_sum(float v) {
+  __shared__ float scratch[32], slots[CTAS];
+  const float own = block_sum(v, scratch);
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+  uint32_t rank;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  if (threadIdx.x < CTAS) {
+    uint32_t at;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(&slots[rank])), "r"(threadIdx.x));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(own) : "memory");
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  float t = 0.f;
+#pragma unroll
+  for (int i = 0; i < CTAS; ++i) t += *reinterpret_cast<volatile float*>(&slots[i]);
+  return t;
+}
+
 // Eight consecutive elements as float32 (two 16-byte loads of float32, one of bfloat16).
 template <typename T> struct Vec8;
 template <> struct Vec8<float> {

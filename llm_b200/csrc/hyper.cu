@@ -164,6 +164,62 @@ hc_norm_vec_kernel(float* __restrict__ resid, MaybePartial<T> y, const float* __
   }
 }
 
+// The same for few rows in bfloat16: a token over a cluster of four CTAs, two columns of every stream a thread, which stay in registers.  One CTA a
+// token is bound by one SM's way to L2 (64 KB both ways at four streams of 2,048) and by 160 multiply-adds a thread.  Float32 rows,
+// whose sums do not depend on how many rows there are, never come here.  8 rows inside decode steps: 7.3 -> 2.6 us a launch; the norm of one stream
+// over the unsummed terms of a product (add_rmsnorm, 64 rows) gained nothing this way (3.4, 3.6 us).
+constexpr int HC_CTAS = 4;
+
+template <int S>
+__global__ void __launch_bounds__(256)
+hc_norm_cluster_kernel(float* __restrict__ resid, MaybePartial<__nv_bfloat16> y, const float* __restrict__ write_mix,
+                       const float* __restrict__ write_out, const float* __restrict__ read_in, const float* __restrict__ gain,
+                       __nv_bfloat16* __restrict__ out, int hidden, float eps) {
+  pdl_launch_dependents();
+  if (out) cluster_begin();
+  const bool pending = write_mix != nullptr;
+  const int c = ((blockIdx.x % HC_CTAS) * blockDim.x + threadIdx.x) * 2, t = blockIdx.x / HC_CTAS;
+  const bool mine = c < hidden;
+  float mix[S][S], wout[S], win[S];
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+    wout[s] = pending ? write_out[s] : 0.f;
+    win[s] = out ? read_in[s] : 0.f;
+#pragma unroll
+    for (int to = 0; to < S; ++to) mix[s][to] = pending ? write_mix[s * S + to] : 0.f;
+  }
+  const float g = out ? gain[0] : 0.f;
+  pdl_wait();
+  float* row = resid + (size_t)t * hidden * S + c;
+  float2 x[S], u = make_float2(0.f, 0.f);
+  if (mine) {
+#pragma unroll
+    for (int s = 0; s < S; ++s) x[s] = *reinterpret_cast<const float2*>(row + (size_t)s * hidden);
+    if (pending) {
+      const float2 yv = make_float2(y.at((size_t)t * hidden + c), y.at((size_t)t * hidden + c + 1));
+      float2 xn[S];
+#pragma unroll
+      for (int to = 0; to < S; ++to) {
+        float2 a = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int s = 0; s < S; ++s) { a.x = fmaf(mix[s][to], x[s].x, a.x); a.y = fmaf(mix[s][to], x[s].y, a.y); }
+        a.x = fmaf(wout[to], yv.x, a.x);
+        a.y = fmaf(wout[to], yv.y, a.y);
+        xn[to] = a;
+        *reinterpret_cast<float2*>(row + (size_t)to * hidden) = a;
+      }
+#pragma unroll
+      for (int s = 0; s < S; ++s) x[s] = xn[s];
+    }
+    if (out)
+#pragma unroll
+      for (int s = 0; s < S; ++s) { u.x = fmaf(win[s], x[s].x, u.x); u.y = fmaf(win[s], x[s].y, u.y); }
+  }
+  if (!out) return;                                // the whole grid, as `out` is the launch's
+  const float r = 1.f / sqrtf(cluster_sum<HC_CTAS>(u.x * u.x + u.y * u.y) / (float)hidden + eps) * g;
+  if (mine) *reinterpret_cast<__nv_bfloat162*>(out + (size_t)t * hidden + c) = __floats2bfloat162_rn(u.x * r, u.y * r);
+}
+
 __global__ void hc_gather_sum_kernel(float* __restrict__ out, const float* __restrict__ resid, const int* __restrict__ rows,
                                      int hidden, int streams) {
   pdl_launch_dependents();
@@ -222,6 +278,16 @@ LLMK_API int llmk_hc_norm(float* resid, const void* y, const float* partials, in
     const size_t smem = (size_t)hidden * sizeof(float);
     const bool vec = hidden % 8 == 0 && (uintptr_t)resid % 16 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)partials % 16 == 0 &&
                      split_stride % 4 == 0 && (uintptr_t)out % 16 == 0;
+    if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+      if (vec && n_tokens * HC_CTAS <= 2 * llmk_sm_count() && streams <= 4 && hidden >= 1024 && hidden <= HC_CTAS * 256 * 2) {
+        auto kern = streams == 1 ? hc_norm_cluster_kernel<1> : streams == 2 ? hc_norm_cluster_kernel<2> : streams == 3 ? hc_norm_cluster_kernel<3>
+                                                                                                        : hc_norm_cluster_kernel<4>;
+        const int threads = ((hidden + HC_CTAS * 2 - 1) / (HC_CTAS * 2) + 31) / 32 * 32;
+        launch_clusters(kern, dim3(n_tokens * HC_CTAS), dim3(threads), HC_CTAS, stream, resid, yy, write_mix, write_out, read_in, gain, (T*)out, hidden,
+                        eps);
+        LLMK_LAUNCH_CHECK("hc_norm");
+      }
+    }
 #define LLMK_HC_VEC(S)                                                                                                  \
   case S:                                                                                                               \
     if (smem > 48 * 1024)                                                                                               \
