@@ -59,7 +59,7 @@ __device__ __forceinline__ void sts(uint32_t at, float v) { asm volatile("st.sha
 
 constexpr int FEW_MAX_STAGES = 16;
 
-enum : int { FEW_OUT_F32 = 0, FEW_OUT_BF16 = 1, FEW_OUT_ADD = 2, FEW_OUT_SILU = 3, FEW_OUT_RELU = 4 };
+enum : int { FEW_OUT_F32 = 0, FEW_OUT_BF16 = 1, FEW_OUT_ADD = 2, FEW_OUT_SILU = 3, FEW_OUT_RELU = 4, FEW_OUT_CLAMPED = 5 };
 
 struct FewArgs {
   const __nv_bfloat16* a;      // rows, or
@@ -72,6 +72,8 @@ struct FewArgs {
   int M, N, K;                 // N: outputs (gated: half the weight rows)
   int tile;                    // weight rows of a tile (gated: gate rows, as many up rows), up to 16 (8)
   int tiles, stages, boxes;    // boxes: of a step
+  const float* bias;           // of the weight rows, or null
+  float limit, alpha;          // of the clamped unit
   int early;                   // steps that are asked for before the rows
   int* error;
 };
@@ -86,7 +88,7 @@ inline int few_rest(int M, int K, bool normed) {
 template <int OUT, bool KEEP>
 __global__ void __launch_bounds__(FEW_WARPS * 32 + 32)
 few_rows_kernel(const __grid_constant__ CUtensorMap weights, const __grid_constant__ CUtensorMap weights_tail, const FewArgs p) {
-  constexpr bool GATED = OUT == FEW_OUT_SILU || OUT == FEW_OUT_RELU;
+  constexpr bool GATED = OUT >= FEW_OUT_SILU;
   pdl_launch_dependents();
   extern __shared__ __align__(1024) unsigned char smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = lane >> 2, quad = lane & 3;
@@ -260,6 +262,8 @@ few_rows_kernel(const __grid_constant__ CUtensorMap weights, const __grid_consta
     const int n0 = min(tile * p.tile, p.N - p.tile), n = n0 + out_row;
     const bool mine = out_token < p.M && n >= tile * p.tile && out_row < p.tile;
     float before = 0.f;
+    float bias = 0.f, bias_up = 0.f;
+    if (p.bias && mine) { bias = p.bias[n]; if (GATED) bias_up = p.bias[p.N + n]; }
     if (OUT == FEW_OUT_ADD && mine) before = reinterpret_cast<float*>(p.out)[(size_t)out_token * p.ldo + n];
     float c[2][4] = {};
     auto release = [&]() {
@@ -320,11 +324,15 @@ few_rows_kernel(const __grid_constant__ CUtensorMap weights, const __grid_consta
         z += lds(get + i * FEW_RED * 4);
         if (GATED) u += lds(get + (i * FEW_RED + 8) * 4);
       }
-      z *= scale; u *= scale;
+      z = fmaf(z, scale, bias); u = fmaf(u, scale, bias_up);
       const size_t at = (size_t)out_token * p.ldo + n;
       if (OUT == FEW_OUT_ADD) z += before;
       if (OUT == FEW_OUT_SILU) z = z / (1.f + expf(-z)) * u;
       if (OUT == FEW_OUT_RELU) z = fmaxf(z, 0.f) * u;
+      if (OUT == FEW_OUT_CLAMPED) {
+        z = fminf(z, p.limit);
+        z = z / (1.f + expf(-p.alpha * z)) * (fminf(fmaxf(u, -p.limit), p.limit) + 1.f);
+      }
       if (OUT == FEW_OUT_F32 || OUT == FEW_OUT_ADD) reinterpret_cast<float*>(p.out)[at] = z;
       else reinterpret_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(z);
     }
@@ -363,7 +371,7 @@ int launch_few(const CUtensorMap& map, const CUtensorMap& tail, const FewArgs& p
   void (*kern)(CUtensorMap, CUtensorMap, FewArgs) =
       out_kind == FEW_OUT_F32 ? few_rows_kernel<FEW_OUT_F32, KEEP> : out_kind == FEW_OUT_BF16 ? few_rows_kernel<FEW_OUT_BF16, KEEP>
       : out_kind == FEW_OUT_ADD ? few_rows_kernel<FEW_OUT_ADD, KEEP> : out_kind == FEW_OUT_SILU ? few_rows_kernel<FEW_OUT_SILU, KEEP>
-      : few_rows_kernel<FEW_OUT_RELU, KEEP>;
+      : out_kind == FEW_OUT_RELU ? few_rows_kernel<FEW_OUT_RELU, KEEP> : few_rows_kernel<FEW_OUT_CLAMPED, KEEP>;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return llmk_fail((int)e, "gemm_few: %s", cudaGetErrorString(e));
@@ -386,17 +394,19 @@ LLMK_API int llmk_gemm_few_supported(int M, int K) {
 }
 
 // out = rows @ w^T.  rows: a (bfloat16) or, with a null, the float32 rows x under an RMS norm with `gain` and `eps`.  out_kind: 0 float32,
-// 1 bfloat16, 2 added to float32 out, 3 / 4 silu / relu of the first N weight rows' product times that of the N behind them, bfloat16.
+// 1 bfloat16, 2 added to float32 out, 3 / 4 silu / relu of the first N weight rows' product times that of the N behind them, bfloat16;
+// 5 the clamped unit of the two, g = min(., limit), g sigmoid(alpha g) (clamp(., -limit, limit) + 1).  bias: float32, one per weight row, or null.
 LLMK_API int llmk_gemm_few(const void* a, const float* x, const float* gain, float eps, long long lda, const void* w, long long ldw, void* out,
-                           long long ldo, int M, int N, int K, int out_kind, cudaStream_t stream) {
+                           long long ldo, int M, int N, int K, int out_kind, const float* bias, float limit, float alpha, cudaStream_t stream) {
   if (M == 0 || N == 0) return 0;
   LLMK_REQUIRE(M > 0 && N > 0 && llmk_gemm_few_supported(M, K), "gemm_few: M=%d N=%d K=%d", M, N, K);
   LLMK_REQUIRE(lda >= K && ldw >= K && ldo >= N && ldw % 8 == 0 && (uintptr_t)w % 16 == 0, "gemm_few: strides %lld %lld %lld", lda, ldw, ldo);
   LLMK_REQUIRE((a != nullptr) != (x != nullptr) && (!a || (lda % 8 == 0 && (uintptr_t)a % 16 == 0)) &&
                (!x || (lda % 4 == 0 && (uintptr_t)x % 16 == 0 && gain && (uintptr_t)gain % 16 == 0)), "gemm_few: rows of one kind, 16-byte aligned");
-  LLMK_REQUIRE(out_kind >= 0 && out_kind <= 4, "gemm_few: unknown output kind %d", out_kind);
+  LLMK_REQUIRE(out_kind >= 0 && out_kind <= 5, "gemm_few: unknown output kind %d", out_kind);
   const bool gated = out_kind >= FEW_OUT_SILU;
   FewArgs p = {(const __nv_bfloat16*)a, x, gain, eps, 1.f / K, lda, out, ldo, M, N, K};
+  p.bias = bias; p.limit = limit; p.alpha = alpha;
   p.error = llmk_error_word(1);
   LLMK_REQUIRE(p.error, "gemm_few: no error word");
   const int sms = llmk_sm_count(), most = gated ? 8 : 16;

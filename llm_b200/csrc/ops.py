@@ -2010,7 +2010,7 @@ def gemm_fast(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, rows: int, pl
 GEMM_FEW = True
 FEW_ROWS = 8
 _FEW_SMEM = 227 * 1024
-_FEW_KINDS = {"add": 2, "silu": 3, "relu": 4}
+_FEW_KINDS = {"add": 2, "silu": 3, "relu": 4, "clamped": 5}
 
 
 @functools.lru_cache(maxsize=4096)
@@ -2029,13 +2029,15 @@ def gemm_few_available(a, w: torch.Tensor, rows: int) -> bool:
     return a.dtype == torch.bfloat16 and a.is_cuda and a.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0
 
 
-def gemm_few(a, w: torch.Tensor, out: torch.Tensor, rows: int, kind=None) -> torch.Tensor:
+def gemm_few(a, w: torch.Tensor, out: torch.Tensor, rows: int, kind=None, bias=None, limit: float = 0.0, alpha: float = 0.0) -> torch.Tensor:
     """out[:rows] = a[:rows] @ w.T for up to 8 rows (gemm_few.cu): every output is one sum, nothing is left to be added up.  a: bfloat16
     rows or NormedRows.  kind None: written in out's dtype; "add": added to float32 out; "silu" or "relu": w = [gate; up] stacked,
-    act(a @ gate.T) * (a @ up.T) in bfloat16."""
+    act(a @ gate.T) * (a @ up.T) in bfloat16; "clamped": the same with the clamped unit (see clamped_glu) of limit and alpha.  bias: float32, one
+    number per row of w, added to the sums."""
     _rows_contig(w, "w"); _rows_contig(out, "out")
     n, k = w.shape
-    n = n // 2 if kind in ("silu", "relu") else n
+    n = n // 2 if kind in ("silu", "relu", "clamped") else n
+    assert bias is None or (bias.dtype == torch.float32 and bias.is_contiguous() and bias.numel() == w.shape[0])
     assert out.shape[1] == n and out.shape[0] >= rows and (kind is None or out.dtype == (torch.float32 if kind == "add" else torch.bfloat16))
     if isinstance(a, NormedRows):
         assert a.resid.dtype == a.gain.dtype == torch.float32 and a.resid.shape[1] == k == a.gain.numel() and rows == a.rows
@@ -2047,7 +2049,7 @@ def gemm_few(a, w: torch.Tensor, out: torch.Tensor, rows: int, kind=None) -> tor
         src = (_ptr(a), c_void_p(0), c_void_p(0), c_float(0.0), c_longlong(a.stride(0)))
     code = _FEW_KINDS[kind] if kind else int(out.dtype == torch.bfloat16)
     _check_t(load_tensor().llmk_gemm_few(*src, _ptr(w), c_longlong(w.stride(0)), _ptr(out), c_longlong(out.stride(0)), c_int(rows), c_int(n),
-                                         c_int(k), c_int(code), _stream()))
+                                         c_int(k), c_int(code), _ptr(bias), c_float(limit), c_float(alpha), _stream()))
     return out
 
 
@@ -2190,7 +2192,7 @@ _ATTN_WAITS = {11: "the query tile", 12: "a key/value tile", 13: "the scores", 1
 def describe_wait(word: int, code: int) -> str:
     """What a code in an error word (1: tensor-core product, 2: tensor-core attention) stands for."""
     if word == 1:
-        kernel = {0: "one-tile", 1: "persistent", 2: "pair"}.get((code - 1) // 3, "unknown")
+        kernel = {0: "one-tile", 1: "persistent", 2: "pair", 3: "few-row"}.get((code - 1) // 3, "unknown")
         return f"the tensor-core product ({kernel} kernel): its {_WAIT_NAMES[code % 3]} gave up a bounded wait (code {code})"
     if word == 2:
         return f"the tensor-core attention gave up a bounded wait for {_ATTN_WAITS.get(code, 'code ' + str(code))} (code {code})"

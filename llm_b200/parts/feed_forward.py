@@ -172,11 +172,14 @@ class ClampedGLU(Part):
     def forward(self, x: torch.Tensor, ctx) -> torch.Tensor:
         T, ws = ctx.n_tokens, ctx.workspace
         I = self.intermediate_size
-        # one product for gate and up; its split-K partial results go unsummed to the activation kernel, which
-        # adds the biases, clamps and multiplies in float32
-        gate_up = linear(x, self.w_gate_up, ws.get("gate_up", T, 2 * I, self.dtype), T, allow_partial=FUSE_PARTIALS)
         act = ws.get("ffn_act", T, I, self.dtype)
-        ops.clamped_glu(act, gate_up, self.b_gate_up, T, self.limit, self.alpha)
+        if T and ops.gemm_few_available(x, self.w_gate_up, T):      # few rows: the unit in the product's epilogue
+            ops.gemm_few(x, self.w_gate_up, act, T, kind="clamped", bias=self.b_gate_up, limit=self.limit, alpha=self.alpha)
+        else:
+            # one product for gate and up; its split-K partial results go unsummed to the activation kernel, which
+            # adds the biases, clamps and multiplies in float32
+            gate_up = linear(x, self.w_gate_up, ws.get("gate_up", T, 2 * I, self.dtype), T, allow_partial=FUSE_PARTIALS)
+            ops.clamped_glu(act, gate_up, self.b_gate_up, T, self.limit, self.alpha)
         return linear(act, self.w_down, ws.get("ffn_out", T, self.hidden_size, self.dtype), T, allow_partial=FUSE_PARTIALS,
                       bias=self.b_down)
 

@@ -76,6 +76,27 @@ def test_rows_under_a_norm(ops, M, N, K):
     assert bool(((out.double() - h @ w.double().T).abs() <= (2.0 ** -9 + 1e-5) * scale).all())
 
 
+@pytest.mark.parametrize("M", [1, 8])
+@pytest.mark.parametrize("N,K", [(34, 64), (2370, 576), (1408, 2048)])
+@pytest.mark.parametrize("biased", [False, True])
+def test_clamped_unit_and_biases(ops, M, N, K, biased):
+    a, w = operands(M, 2 * N, K)
+    bias = torch.randn(2 * N, device=DEV) if biased else None
+    z = a.double() @ w.double().T + (bias.double() if biased else 0)
+    scale = a.double().abs() @ w.double().abs().T
+    limit, alpha = 1.5, 1.702
+    g, u = z[:, :N].clamp(max=limit), z[:, N:].clamp(-limit, limit)
+    ref = g * torch.sigmoid(alpha * g) * (u + 1)
+    out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    ops.gemm_few(a, w, out, M, kind="clamped", bias=bias, limit=limit, alpha=alpha)
+    # slopes: the gate's function of at most 1.1 in the range that is clamped above, the linear branch's factor of at most 2.5
+    slack = 2.0 ** -8 * ref.abs() + 3 * BOUND * (scale[:, :N] + scale[:, N:] * g.abs()) + 1e-6
+    assert bool(((out.double() - ref).abs() <= slack).all())
+    rows = torch.empty(M, 2 * N, device=DEV)
+    ops.gemm_few(a, w, rows, M, bias=bias)
+    assert bool(((rows.double() - z).abs() <= BOUND * (scale + 1)).all())
+
+
 def test_what_is_not_taken(ops):
     a, w = operands(8, 64, 128)
     assert not ops.gemm_few_available(a.float(), w.float(), 8)
