@@ -380,7 +380,9 @@ int launch_few(const CUtensorMap& map, const CUtensorMap& tail, const FewArgs& p
   LLMK_LAUNCH_CHECK("gemm_few");
 }
 
-constexpr int FEW_SMEM = 227 * 1024, FEW_LEAST_STAGES = 3;
+// What must be left beside the rows, in boxes: 8 rows of 8,448 leave room for three, and the tcgen05 kernel's swapped mode is ahead then (a call of the
+// design with that width 21.50 ms against 21.58); 3 rows of 14,336 leave four, and a decode step takes 3,198 us against 3,253.
+constexpr int FEW_SMEM = 227 * 1024, FEW_LEAST_STAGES = 4;
 // The most that is in flight, and how much of it is asked for before the rows, which wait behind that.  Decode steps of 1.1 B (1, 4, 8 rows), all of the
 // ring first: 64 KB 771, 795, 828 us; 100 KB 695, 712, 746; 140 KB 666, 690, 750; 200 KB 677, 719, 755 (649, 675, 738 with 140 KB once the rows
 // were kept in registers); of 140 KB first 96 KB: 634, 665, 717; 72 KB: 629, 667, 716; 57 KB: 638, 668, 727.

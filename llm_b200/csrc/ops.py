@@ -2017,7 +2017,7 @@ _FEW_KINDS = {"add": 2, "silu": 3, "relu": 4, "clamped": 5}
 def gemm_few_takes(rows: int, k: int) -> bool:
     """Whether the few-row product takes so many rows of k channels (as llmk_gemm_few_supported)."""
     rest = k * rows * 2 + 4 * k + 2 * 8 * 160 * 4 + 256 + 34 * 8
-    return 0 < rows <= FEW_ROWS and k > 0 and k % 64 == 0 and rest + 3 * 16384 <= _FEW_SMEM
+    return 0 < rows <= FEW_ROWS and k > 0 and k % 64 == 0 and rest + 4 * 16384 <= _FEW_SMEM
 
 
 def gemm_few_available(a, w: torch.Tensor, rows: int) -> bool:
