@@ -238,7 +238,7 @@ class PagedAttention(Part):
                               k_pages.shape[1], self.head_dim, self.window or 0, self.scale,
                               write_kv=not self.shares_cache,
                               q_rot=lambda: ws.get("q_rot", T, self.q_size, self.dtype))
-        if into is not None and self.b_o is None and linear_add(attn, self.w_o, into.resid, T):
+        if into is not None and self.b_o is None and linear_add(attn, self.w_o, into, T):
             return None
         return linear(attn, self.w_o, ws.get("mixer_out", T, self.hidden_size, self.dtype), T,
                       allow_partial=FUSE_PARTIALS and not whole, bias=self.b_o)
@@ -274,7 +274,7 @@ class PagedAttention(Part):
                             value_dim=V, softcap=self.softcap, sink=self.sink, keep_first=self.keep_first,
                             chunk=self.chunk, sigmoid_bias=self.score_bias, sink_values=self.sink_values,
                             dist_bias=(self.r1, self.r2) if self.dist_bias else None)
-        if into is not None and linear_add(attn, self.w_o, into.resid, T):
+        if into is not None and linear_add(attn, self.w_o, into, T):
             return None
         return linear(attn, self.w_o, ws.get("mixer_out", T, self.hidden_size, self.dtype), T, allow_partial=FUSE_PARTIALS and not whole)
 

@@ -92,7 +92,7 @@ class DifferentialAttention(Part):
         gate = proj[:, self.q_size + self.k_size + self.v_size:] if self.gated else None
         out = ws.get("attn_out", T, self.o_size, self.dtype)
         ops.diff_combine(out, maps, gate, T, H, self.per_group, self.lam, 1.0 - self.diff, self.eps)
-        if into is not None and linear_add(out, self.w_o, into.resid, T):
+        if into is not None and linear_add(out, self.w_o, into, T):
             return None
         return linear(out, self.w_o, ws.get("mixer_out", T, self.hidden_size, self.dtype), T, allow_partial=FUSE_PARTIALS)
 

@@ -69,7 +69,7 @@ class SwiGLU(Part):
             gate_up = linear(x, self.w_gate_up, ws.get("gate_up", T, 2 * self.intermediate_size, self.dtype), T,
                              allow_partial=FUSE_PARTIALS, bias=self.b_gate_up)
             ops.silu_mul(act, gate_up, T, self.activation)
-        if into is not None and self.b_down is None and linear_add(act, self.w_down, into.resid, T):
+        if into is not None and self.b_down is None and linear_add(act, self.w_down, into, T):
             return None
         return linear(act, self.w_down, ws.get(tag + "_out", T, self.hidden_size, self.dtype), T, allow_partial=FUSE_PARTIALS,
                       bias=self.b_down)
@@ -128,7 +128,7 @@ class ActMLP(Part):
         if not linear_act(x, self.w_up, act, T, self.activation):      # many rows: the activation in the product's epilogue
             up = linear(x, self.w_up, ws.get(tag + "_up", T, self.intermediate_size, self.dtype), T, allow_partial=FUSE_PARTIALS)
             ops.act_rows(act, up, T, self.activation)
-        if into is not None and linear_add(act, self.w_down, into.resid, T):
+        if into is not None and linear_add(act, self.w_down, into, T):
             return None
         return linear(act, self.w_down, ws.get(tag + "_out", T, self.hidden_size, self.dtype), T, allow_partial=FUSE_PARTIALS)
 

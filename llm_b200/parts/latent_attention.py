@@ -210,7 +210,7 @@ class LatentAttention(Part):
                             sink_values=self.sink_values)
         attn = ws.get("attn_out", T, H * self.value_dim, self.dtype)
         ops.gemm_heads(o_lat, self.w_uv, attn, T, H)
-        if into is not None and linear_add(attn, self.w_o, into.resid, T):
+        if into is not None and linear_add(attn, self.w_o, into, T):
             return None
         return linear(attn, self.w_o, ws.get("mixer_out", T, self.hidden_size, self.dtype), T, allow_partial=FUSE_PARTIALS)
 
@@ -232,7 +232,7 @@ class LatentAttention(Part):
         ops.paged_attention(o_lat, q_lat, pages, pages, view.group, ctx, H, 1, RW, 0, self.scale)
         attn = ws.get("attn_out", T, H * self.value_dim, self.dtype)
         ops.gemm_heads(o_lat, self.w_uv, attn, T, H, gate=gate)
-        if into is not None and linear_add(attn, self.w_o, into.resid, T):
+        if into is not None and linear_add(attn, self.w_o, into, T):
             return None
         return linear(attn, self.w_o, ws.get("mixer_out", T, self.hidden_size, self.dtype), T, allow_partial=FUSE_PARTIALS)
 

@@ -11,6 +11,7 @@ from __future__ import annotations
 import torch
 
 from ..csrc import ops
+from .base import ResidualStream
 
 
 # Whether the built-in parts hand split-K partial results to the next kernel instead of summing
@@ -46,12 +47,14 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, rows: int, 
     return res
 
 
-def linear_add(x: torch.Tensor, weight: torch.Tensor, resid: torch.Tensor, rows: int) -> bool:
-    """resid[:rows] += x[:rows] @ weight.T, float32, in the product's epilogue.  Returns False, having done nothing, where there are more rows
-    than the few-row product takes (or float32 operands): the caller then leaves the sum to the next norm."""
+def linear_add(x: torch.Tensor, weight: torch.Tensor, stream: ResidualStream, rows: int) -> bool:
+    """stream.resid[:rows] += x[:rows] @ weight.T, float32, in the product's epilogue; the stream's rows in the compute dtype are then no longer
+    those of resid, and are dropped.  Returns False, having done nothing, where there are more rows than the few-row product takes (or float32
+    operands): the caller then leaves the sum to the next norm."""
     if rows == 0 or not ops.gemm_few_available(x, weight, rows):
         return rows == 0
-    ops.gemm_few(x, weight, resid, rows, kind="add")
+    ops.gemm_few(x, weight, stream.resid, rows, kind="add")
+    stream.rows_cast = None
     return True
 
 
