@@ -155,7 +155,8 @@ class ResidualStream:
         # a pending term that is still to be normed and scaled before it joins the residual:
         # (the norm part that does it, multiplier); None: the term is added as it is
         self.pending_post = None
-        # the stream's rows in the compute dtype, while they are those of resid (kept by norms that stand behind the sum)
+        # the stream's rows in the compute dtype, while they are those of resid (kept by norms that stand behind the sum;
+        # dropped by fold, by products that add to resid and behind a transform of the whole stream)
         self.rows_cast: Optional[torch.Tensor] = None
 
     def as_rows(self, ctx, dtype: torch.dtype) -> torch.Tensor:
@@ -172,6 +173,7 @@ class ResidualStream:
         """Add what is pending, so that resid is the whole stream."""
         if self.pending is None:
             return
+        self.rows_cast = None
         if self.pending_post is not None:
             self.pending_post[0].fold(self, ctx)
         else:

@@ -140,9 +140,7 @@ class PostNormBlock:
 
     def forward(self, stream: ResidualStream, ctx, view) -> None:
         p = self.parts
-        if stream.pending is not None:
-            stream.fold(ctx)
-            stream.rows_cast = None
+        stream.fold(ctx)
         p["norm1"].close(stream, self.mixer.forward(stream.as_rows(ctx, self.dtype), ctx, view), self.alpha, ctx)
         if self.ffn is not None:
             p["norm2"].close(stream, self.ffn.forward(stream.as_rows(ctx, self.dtype), ctx, **self.unsummed), self.alpha, ctx)
@@ -162,6 +160,7 @@ class StreamBlock:
 
     def forward(self, stream: ResidualStream, ctx, view) -> None:
         self.parts["stream"].forward(stream, ctx)
+        stream.rows_cast = None
 
 
 register_part("block", "stream", StreamBlock)

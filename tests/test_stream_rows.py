@@ -73,8 +73,8 @@ class Scaled:
 
 def layers(device, tensors):
     from llm_b200.models.spec import PartSpec
-    from llm_b200.parts.base import build_part, part_class, register_part
-    from llm_b200.parts.block import PostNormBlock, PreNormBlock
+    from llm_b200.parts.base import part_class, register_part
+    from llm_b200.parts.block import PostNormBlock, PreNormBlock, StreamBlock
     try:
         part_class("mixer", "scaled_rows")
     except KeyError:
@@ -84,9 +84,9 @@ def layers(device, tensors):
     post = [PostNormBlock({"mixer": mixer, "norm1": norm(f"post{i}")}, BF16, device, alpha=ALPHA) for i in (0, 1)]
     pre = PreNormBlock({"norm1": norm("n1"), "mixer": mixer, "norm2": norm("n2"),
                         "ffn": PartSpec("swiglu", {"hidden_size": W, "intermediate_size": FF}, "ff")}, BF16, device)
-    again = build_part("stream", PartSpec("embedding_reinjection", {"hidden_size": W, "vocab_size": 32, "passes": 1, "pass_index": 0,
-                                                                    "table_name": "table"}, "loop"), BF16, device)
-    for part in [p for b in post + [pre] for p in b.parts.values() if hasattr(p, "bind")] + [again]:
+    again = StreamBlock({"stream": PartSpec("embedding_reinjection", {"hidden_size": W, "vocab_size": 32, "passes": 1, "pass_index": 0,
+                                                                      "table_name": "table"}, "loop")}, BF16, device)
+    for part in [p for b in post + [pre, again] for p in b.parts.values() if hasattr(p, "bind")]:
         for name, info in part.parameters().items():
             g = torch.Generator().manual_seed(len(tensors))
             t = torch.randn(info.shape, generator=g) * (0.12 if info.kind == "matrix" else 0.1)      # sublayers as large as the stream
@@ -115,7 +115,7 @@ def check(device, rows, middle):
         h = rms(x, "n2")
         x = x + (torch.nn.functional.silu(h @ t["ff.gate_proj.weight"].T) * (h @ t["ff.up_proj.weight"].T)) @ t["ff.down_proj.weight"].T
     if "stream" in middle:
-        again.forward(stream, ctx)
+        again.forward(stream, ctx, None)
         x = torch.cat([x, t["table"][ids.long()]], -1) @ t["loop.in"].T + t["loop.step"][0]
     post[1].forward(stream, ctx, None)
     x = rms((ALPHA + 0.75) * x, "post1")
@@ -124,7 +124,7 @@ def check(device, rows, middle):
     assert float((stream.resid.to(F64) - x).norm() / x.norm()) < 0.03
 
 
-@pytest.mark.parametrize("middle", ["prenorm"])
+@pytest.mark.parametrize("middle", ["prenorm", "stream", "prenorm stream"])
 @pytest.mark.parametrize("rows", [4, 8, 9, 12])
 def test_rows_after_other_arrangements(rows, middle, monkeypatch):
     plain_kernels(monkeypatch)
@@ -132,7 +132,7 @@ def test_rows_after_other_arrangements(rows, middle, monkeypatch):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("middle", ["prenorm"])
+@pytest.mark.parametrize("middle", ["prenorm", "stream", "prenorm stream"])
 @pytest.mark.parametrize("rows", [4, 8, 9, 12])
 def test_rows_after_other_arrangements_on_the_kernels(rows, middle):
     check(torch.device("cuda"), rows, middle)
