@@ -162,8 +162,9 @@ paged_attention_generic_kernel(T* __restrict__ out, long long out_stride, const 
       p = valid ? 1.f / (1.f + expf(-(s + bias))) : 0.f;
     } else {
       const float m_new = fmaxf(m, warp_max(s));
-      const float alpha = expf(m - m_new);  // m = -inf at the first tile gives 0
-      p = valid ? expf(s - m_new) : 0.f;
+      // a score of -inf weighs nothing, also in a first tile that holds no other (a warp's first, where four share a head): -inf - -inf is NaN
+      const float alpha = m_new == -INFINITY ? 1.f : expf(m - m_new);
+      p = valid && s != -INFINITY ? expf(s - m_new) : 0.f;
       l = l * alpha + warp_sum(p);
       m = m_new;
 #pragma unroll
@@ -193,7 +194,8 @@ paged_attention_generic_kernel(T* __restrict__ out, long long out_stride, const 
     }
   }
   if (SPLIT > 1) {
-    // the parts' sums, in the order of the warps, against the largest of their maxima (a warp without a tile: -inf, weight 0)
+    // the parts' sums, in the order of the warps, against the largest of their maxima (a warp without a tile, or with scores of -inf alone: -inf,
+    // weight 0).  The values of a part of weight 0 are left out, as those of a key of weight 0 are: an infinite one would make a NaN.
     __shared__ float m_s[WARPS], l_s[WARPS], acc_s[WARPS][MAXD];
     if (lane == 0) { m_s[warp] = m; l_s[warp] = l; }
 #pragma unroll
@@ -210,8 +212,9 @@ paged_attention_generic_kernel(T* __restrict__ out, long long out_stride, const 
     for (int w = 0; w < SPLIT; ++w) {
       const float f = gated ? 1.f : expf(m_s[warp + w] - all);
       l += l_s[warp + w] * f;
+      if (f != 0.f)
 #pragma unroll
-      for (int i = 0; i < MAXD / 32; ++i) acc[i] += acc_s[warp + w][lane + 32 * i] * f;
+        for (int i = 0; i < MAXD / 32; ++i) acc[i] += acc_s[warp + w][lane + 32 * i] * f;
     }
   }
   const float inv = gated ? 1.f : 1.f / l;

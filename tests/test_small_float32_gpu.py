@@ -54,3 +54,88 @@ def test_general_attention_over_head_sizes(ops, HS, n, window):
         ops.paged_attention_generic(last, q[-1:], kp, vp, bt.to(DEV), torch.zeros(1, dtype=torch.int32, device=DEV),
                                     i[-1:].to(torch.int32).contiguous(), 1, NH, NKV, HS, window, 1.0 / math.sqrt(HS))
         assert torch.equal(last[0], out[-1])
+
+
+def attend(q, k, v, seen, scale, sink=None, gate=None):
+    """One query a row in 64 bits: q [t, h, d], k [j, d], v [j, e], seen [t, j]; sink: score per head without a value; gate: sigmoid weights."""
+    s = torch.einsum("thd,jd->htj", q, k) * scale
+    s = s.masked_fill(~seen, -math.inf)
+    if gate is not None:
+        p = torch.sigmoid(s + gate[:, None, None])
+    else:
+        p = torch.softmax(s if sink is None else torch.cat([s, sink[:, None, None].expand(-1, s.shape[1], 1)], -1), -1)[..., :k.shape[0]]
+    return torch.einsum("htj,je->the", p, torch.where(seen.any(0)[:, None], v, 0.0)).flatten(1)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("HS", [32, 64, 128])
+@pytest.mark.parametrize("n,option", [(33, ""), (161, ""), (161, "sink"), (161, "learned"), (161, "keep"), (300, "keep"), (161, "chunk"), (300, "chunk"),
+                                      (161, "sigmoid"), (300, "sigmoid")])
+@pytest.mark.parametrize("lowest", ["none", "last key", "a tile", "first tile"])
+def test_general_attention_with_options_and_scores_of_minus_infinity(ops, dtype, HS, n, option, lowest):
+    """Up to 64 channels four warps take a head's tiles of 32 keys in turn: options that leave tiles out, and keys whose product with the query is
+    -inf, which weigh nothing wherever they lie (in tiles that hold no other, too); in every form the weights' sums are over what is left."""
+    if lowest == "first tile" and option in ("chunk", "sigmoid"):
+        pytest.skip("the last queries see no key of it")
+    page, NH = 8, 3
+    g = torch.Generator(device=DEV).manual_seed(HS + n)
+    rand = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    pages = -(-n // page)
+    kp, vp = (rand(pages, 1, page, HS).to(dtype) for _ in range(2))
+    q = rand(n, NH * HS).abs().to(dtype)
+    rows = {"none": [], "last key": [n - 1], "a tile": list(range(64, 96)) if n > 96 else [32], "first tile": list(range(32))}[lowest]
+    for j in rows:
+        kp[j // page, 0, j % page, 5] = -math.inf
+    i = torch.arange(n, device=DEV)
+    dist = i[:, None] - i[None]
+    seen = dist >= 0
+    kw, window, sink, gate = {}, 0, None, None
+    if option == "sink":
+        kw, sink = dict(sink=True), torch.zeros(NH, device=DEV).double()
+    if option == "learned":
+        kw = dict(sink=True, sink_values=rand(NH) * 2)
+        sink = kw["sink_values"].double()
+    if option == "keep":
+        window, kw = 40, dict(keep_first=6)
+        seen = seen & ((dist < 40) | (i[None] < 6))
+    if option in ("chunk", "sigmoid"):
+        kw = dict(chunk=150)
+        seen = seen & (i[:, None] // 150 == i[None] // 150)
+    if option == "sigmoid":
+        kw["sigmoid_bias"] = rand(NH) - 2
+        gate = kw["sigmoid_bias"].double()
+    k, v = (p.reshape(-1, HS)[:n].double() for p in (kp, vp))
+    k = torch.where(torch.isinf(k), 0.0, k)
+    low = torch.zeros(n, dtype=torch.bool, device=DEV)
+    low[rows] = True
+    seen = seen & ~low[None]
+    some = seen.any(1) | (option in ("sink", "learned", "sigmoid"))      # the other queries see scores of -inf alone
+    ref = attend(q.double().view(n, NH, HS), k, v, seen, HS ** -0.5, sink, gate)
+    out = torch.empty(n, NH * HS, device=DEV, dtype=dtype)
+    ops.paged_attention_generic(out, q, kp, vp, torch.arange(pages, dtype=torch.int32, device=DEV)[None].contiguous(),
+                                torch.zeros(n, dtype=torch.int32, device=DEV), i.to(torch.int32), n, NH, 1, HS, window, HS ** -0.5, **kw)
+    # float32 sums of n weights and HS products; bfloat16 results are rounded once more
+    assert float((out.double() - ref)[some].norm() / ref[some].norm()) < (2e-6 if dtype == torch.float32 else 2.0 ** -8)
+
+
+@pytest.mark.parametrize("HS", [32, 64, 128])
+def test_infinite_values_of_keys_that_weigh_nothing(ops, HS):
+    """A key 400 below the largest score has the weight exp(-400) = 0 in float32, and its value counts nothing, whichever tile it lies in."""
+    n, page = 161, 8
+    q = torch.zeros(1, HS, device=DEV)
+    q[0, 0] = 1.0
+    kp = torch.zeros(-(-n // page), 1, page, HS, device=DEV)
+    vp = torch.randn_like(kp)
+    for j in (40, 160):
+        kp[j // page, 0, j % page, 0] = -400.0
+        vp[j // page, 0, j % page, 3] = math.inf
+    # a tile of such keys alone, and no other for its warp
+    for j in range(96, 128):
+        kp[j // page, 0, j % page, 0], vp[j // page, 0, j % page, 7] = -400.0, math.inf
+    v = vp.reshape(-1, HS)[:n].double()
+    keep = [j for j in range(n) if j not in (40, 160) and not 96 <= j < 128]
+    out = torch.empty(1, HS, device=DEV)
+    ops.paged_attention_generic(out, q, kp, vp, torch.arange(kp.shape[0], dtype=torch.int32, device=DEV)[None].contiguous(),
+                                torch.zeros(1, dtype=torch.int32, device=DEV), torch.tensor([n - 1], dtype=torch.int32, device=DEV), 1, 1, 1, HS, 0, 1.0)
+    ref = v[keep].mean(0)
+    assert float((out[0].double() - ref).norm() / ref.norm()) < 2e-6
