@@ -1,6 +1,6 @@
 // Causal grouped-query attention over the paged cache, any sizes, float32 arithmetic.
 //
-// One warp owns one (token, query head); up to 64 channels four do.  Keys are visited in tiles of 32 that start
+// One warp owns one (token, query head); up to 64 channels four do while there are few of them.  Keys are visited in tiles of 32 that start
 // at absolute positions 0, 32, 64, ...: lane j scores key tile+j, the warp keeps a
 // running maximum and sum (online softmax), then all lanes add p_j * v_j in key order.
 // The order of every sum is a function of the token's own position alone, so a
@@ -30,8 +30,14 @@ constexpr int WARPS = 4;
 // this way, with the rows asked for ahead.)
 constexpr int MAX_HEAD_DIM = 1024;
 constexpr int PREFETCH_TILES = 4;      // tiles of keys and values that a warp asks into L1 ahead of their turn
-// Small heads: the block's four warps take a head's tiles in turn (which warp follows from a tile's position alone, so the order of a token's
-// sums still does) and their sums are put together at the end: 18.2 -> 5.8 us a launch.
+// Small heads: a head's tiles are dealt to four parts in turn (to which one follows from a tile's position alone, so the order of a token's
+// sums still does) and the parts' sums are put together at the end.  The block's four warps take a part each: 18.2 -> 5.8 us a launch of few
+// requests.  In a launch of many (token, head) pairs (prompts of many short requests) a block's other warps have nothing to take, and a warp
+// takes the four parts after one another instead, the same numbers in the same order.  Where the line lies, in pairs an SM: us a launch in
+// float32, head size 32, one warp a head without parts / four warps / one warp with parts: 4,096 pairs of 8 keys 6.8 / 18.1 / 6.0, of 32 keys
+// 15.5 / 22.3 / 10.9, of 113 keys 47 / 36 / 34, of 1,000 keys 557 / 226 / 238; 2,048 pairs of 8 keys 6.0 / 10.1 / 5.0, of 32 keys 13.2 / 12.2 /
+// 8.0, of 113 keys 42 / 20 / 24, of 1,000 keys 353 / 126 / 171: up to 16 an SM what long contexts gain is more than what the shortest lose.
+constexpr int SERIAL_FROM = 16;
 __host__ __device__ constexpr int split_of(int max_dim) { return max_dim <= 64 ? WARPS : 1; }
 
 template <typename T>
@@ -77,7 +83,7 @@ __device__ __forceinline__ float dot_row_scalar(const float* __restrict__ q, con
   return s;
 }
 
-template <typename T, int MAXD>
+template <typename T, int MAXD, bool SERIAL>
 __global__ void __launch_bounds__(WARPS * 32)
 paged_attention_generic_kernel(T* __restrict__ out, long long out_stride, const T* __restrict__ q,
                                long long q_stride, const T* __restrict__ k_pages,
@@ -89,15 +95,15 @@ paged_attention_generic_kernel(T* __restrict__ out, long long out_stride, const 
                                const float* __restrict__ sigmoid_bias, const float* __restrict__ dist_r1,
                                const float* __restrict__ dist_r2, int v_share) {
   constexpr int AHEAD = MAXD <= 256 ? 8 : MAXD <= 512 ? 4 : 2;
-  constexpr int SPLIT = split_of(MAXD);            // warps that share a (token, head)
+  constexpr int SPLIT = split_of(MAXD);            // parts of a (token, head)
+  constexpr int SHARE = SERIAL ? 1 : SPLIT;        // warps that share them
   __shared__ float q_s[WARPS][MAXD];
   __shared__ __align__(16) float p_s[WARPS][32];
   __shared__ __align__(16) long long row_s[WARPS][32];
   pdl_launch_dependents();      // let the next kernel start its own prologue now
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long item = ((long long)blockIdx.x * WARPS + warp) / SPLIT;
-  const int part = warp % SPLIT;
+  const long long item = ((long long)blockIdx.x * WARPS + warp) / SHARE;
   if (item >= (long long)n_tokens * n_heads) return;
   const int t = (int)(item / n_heads), h = (int)(item % n_heads);
   const int g = h / (n_heads / n_kv);
@@ -106,6 +112,7 @@ paged_attention_generic_kernel(T* __restrict__ out, long long out_stride, const 
   const int lo = chunk > 0 ? (pos / chunk) * chunk : (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
   const int keep_end = min(keep_first, lo);      // keys [0, keep_end) lie before the window and are seen all the same
   const int lo_tile = (lo / 32) * 32;
+  const int used = SERIAL ? max(1, min(SPLIT, (pos >> 5) + 1)) : SPLIT;      // a short context leaves parts without a tile: nothing to merge
   const float inv_cap = softcap > 0.f ? 1.f / softcap : 0.f;
   const float r1 = dist_r1 ? dist_r1[h] : 0.f, r2 = dist_r1 ? dist_r2[h] : 0.f;
   const int n_v = n_kv / v_share, gv = g / v_share;      // v_share neighbouring key heads read one value head
@@ -126,95 +133,105 @@ paged_attention_generic_kernel(T* __restrict__ out, long long out_stride, const 
   };
   const bool ahead = MAXD <= 64 && keep_end == 0;
   if (ahead)
-    for (int i = 0, tile = lo_tile; i < PREFETCH_TILES * SPLIT; ++i, tile += 32)
-      if ((tile >> 5) % SPLIT == part) prefetch_tile(tile);
+    for (int i = 0, tile = lo_tile; i < PREFETCH_TILES * SHARE; ++i, tile += 32)
+      if ((tile >> 5) % SHARE == warp % SHARE) prefetch_tile(tile);
 
-  float acc[MAXD / 32];
-#pragma unroll
-  for (int i = 0; i < MAXD / 32; ++i) acc[i] = 0.f;
-  // the sink is the first term of the softmax: score 0, weight exp(0 - m), no value
   const bool gated = sigmoid_bias != nullptr;
   const float bias = gated ? sigmoid_bias[h] : 0.f;
-  const bool with_sink = sink && part == 0;
-  float m = with_sink ? (sink_values ? sink_values[h] : 0.f) : -INFINITY, l = with_sink ? 1.f : 0.f;
-
-  for (int tile = keep_end > 0 ? 0 : lo_tile; tile <= pos; tile += 32) {
-    if (tile >= keep_end && tile < lo_tile) {      // between the kept keys and the window: nothing to see
-      tile = lo_tile - 32;
-      continue;
-    }
-    if (SPLIT > 1 && (tile >> 5) % SPLIT != part) continue;      // by absolute position, whatever the window's start
-    if (ahead) prefetch_tile(tile + 32 * PREFETCH_TILES * SPLIT);
-    const int kp = tile + lane;
-    const bool valid = kp <= pos && (kp >= lo || kp < keep_end);
-    long long row = 0;                             // the value's place in units of rows of vdim
-    float s = -INFINITY;
-    if (valid) {
-      const int page = table[kp / page_size];
-      row = ((long long)page * n_v + gv) * page_size + kp % page_size;
-      const T* k_row = k_pages + (((long long)page * n_kv + g) * page_size + kp % page_size) * head_dim;
-      s = (vec ? dot_row<T>(q_s[warp], k_row, head_dim) : dot_row_scalar<T>(q_s[warp], k_row, head_dim)) * scale;
-      if (softcap > 0.f) s = softcap * tanhf(s * inv_cap);
-      if (dist_r1) s -= r1 * log1pf(r2 * (float)(pos - kp));      // a bias that grows with the distance to the key
-    }
-    float p;
-    if (gated) {
-      p = valid ? 1.f / (1.f + expf(-(s + bias))) : 0.f;
-    } else {
-      const float m_new = fmaxf(m, warp_max(s));
-      // a score of -inf weighs nothing, also in a first tile that holds no other (a warp's first, where four share a head): -inf - -inf is NaN
-      const float alpha = m_new == -INFINITY ? 1.f : expf(m - m_new);
-      p = valid && s != -INFINITY ? expf(s - m_new) : 0.f;
-      l = l * alpha + warp_sum(p);
-      m = m_new;
-#pragma unroll
-      for (int i = 0; i < MAXD / 32; ++i) acc[i] *= alpha;
-    }
-    // the values of several keys asked for together (a key after the other waits for memory 32 times a tile), added in the keys' order
-    __syncwarp();                                  // the tile before has been read
-    p_s[warp][lane] = p;
-    row_s[warp][lane] = row;
-    __syncwarp();
-    const int n_valid = min(32, pos - tile + 1);
+  float acc[MAXD / 32], m, l;
+  __shared__ float m_s[WARPS / SHARE][SPLIT], l_s[WARPS / SHARE][SPLIT], acc_s[SPLIT > 1 ? WARPS / SHARE : 1][SPLIT][SPLIT > 1 ? MAXD : 1];
+  const int owner = warp / SHARE;                  // of the (token, head) among the block's
 #pragma unroll 1
-    for (int j = 0; j < n_valid; j += AHEAD) {
-      float v[AHEAD][MAXD / 32], pj[AHEAD];
+  for (int part = warp % SHARE; part < used; part += SHARE) {
 #pragma unroll
-      for (int u = 0; u < AHEAD; ++u) {
-        pj[u] = p_s[warp][j + u];                    // 0 for a key past the last (AHEAD divides 32)
-        const T* at = v_pages + row_s[warp][j + u] * vdim;
-#pragma unroll
-        for (int i = 0; i < MAXD / 32; ++i) v[u][i] = pj[u] != 0.f && lane + 32 * i < vdim ? to_f32(at[lane + 32 * i]) : 0.f;
+    for (int i = 0; i < MAXD / 32; ++i) acc[i] = 0.f;
+    // the sink is the first term of the softmax: score 0, weight exp(0 - m), no value
+    const bool with_sink = sink && part == 0;
+    m = with_sink ? (sink_values ? sink_values[h] : 0.f) : -INFINITY;
+    l = with_sink ? 1.f : 0.f;
+
+    for (int tile = keep_end > 0 ? 0 : lo_tile; tile <= pos; tile += 32) {
+      if (tile >= keep_end && tile < lo_tile) {      // between the kept keys and the window: nothing to see
+        tile = lo_tile - 32;
+        continue;
       }
+      if (SPLIT > 1 && (tile >> 5) % SPLIT != part) continue;      // by absolute position, whatever the window's start
+      if (ahead) prefetch_tile(tile + 32 * PREFETCH_TILES * SPLIT);
+      const int kp = tile + lane;
+      const bool valid = kp <= pos && (kp >= lo || kp < keep_end);
+      long long row = 0;                             // the value's place in units of rows of vdim
+      float s = -INFINITY;
+      if (valid) {
+        const int page = table[kp / page_size];
+        row = ((long long)page * n_v + gv) * page_size + kp % page_size;
+        const T* k_row = k_pages + (((long long)page * n_kv + g) * page_size + kp % page_size) * head_dim;
+        s = (vec ? dot_row<T>(q_s[warp], k_row, head_dim) : dot_row_scalar<T>(q_s[warp], k_row, head_dim)) * scale;
+        if (softcap > 0.f) s = softcap * tanhf(s * inv_cap);
+        if (dist_r1) s -= r1 * log1pf(r2 * (float)(pos - kp));      // a bias that grows with the distance to the key
+      }
+      float p;
+      if (gated) {
+        p = valid ? 1.f / (1.f + expf(-(s + bias))) : 0.f;
+      } else {
+        const float m_new = fmaxf(m, warp_max(s));
+        // a score of -inf weighs nothing, also in a first tile that holds no other (a warp's first, where four share a head): -inf - -inf is NaN
+        const float alpha = m_new == -INFINITY ? 1.f : expf(m - m_new);
+        p = valid && s != -INFINITY ? expf(s - m_new) : 0.f;
+        l = l * alpha + warp_sum(p);
+        m = m_new;
 #pragma unroll
-      for (int u = 0; u < AHEAD; ++u)
-        if (pj[u] != 0.f)
+        for (int i = 0; i < MAXD / 32; ++i) acc[i] *= alpha;
+      }
+      // the values of several keys asked for together (a key after the other waits for memory 32 times a tile), added in the keys' order
+      __syncwarp();                                  // the tile before has been read
+      p_s[warp][lane] = p;
+      row_s[warp][lane] = row;
+      __syncwarp();
+      const int n_valid = min(32, pos - tile + 1);
+#pragma unroll 1
+      for (int j = 0; j < n_valid; j += AHEAD) {
+        float v[AHEAD][MAXD / 32], pj[AHEAD];
 #pragma unroll
-          for (int i = 0; i < MAXD / 32; ++i) acc[i] = fmaf(pj[u], v[u][i], acc[i]);
+        for (int u = 0; u < AHEAD; ++u) {
+          pj[u] = p_s[warp][j + u];                    // 0 for a key past the last (AHEAD divides 32)
+          const T* at = v_pages + row_s[warp][j + u] * vdim;
+#pragma unroll
+          for (int i = 0; i < MAXD / 32; ++i) v[u][i] = pj[u] != 0.f && lane + 32 * i < vdim ? to_f32(at[lane + 32 * i]) : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u)
+          if (pj[u] != 0.f)
+#pragma unroll
+            for (int i = 0; i < MAXD / 32; ++i) acc[i] = fmaf(pj[u], v[u][i], acc[i]);
+      }
+    }
+    if (SPLIT > 1) {
+      if (lane == 0) { m_s[owner][part] = m; l_s[owner][part] = l; }
+#pragma unroll
+      for (int i = 0; i < MAXD / 32; ++i) acc_s[owner][part][lane + 32 * i] = acc[i];
     }
   }
   if (SPLIT > 1) {
-    // the parts' sums, in the order of the warps, against the largest of their maxima (a warp without a tile, or with scores of -inf alone: -inf,
-    // weight 0).  The values of a part of weight 0 are left out, as those of a key of weight 0 are: an infinite one would make a NaN.
-    __shared__ float m_s[WARPS], l_s[WARPS], acc_s[WARPS][MAXD];
-    if (lane == 0) { m_s[warp] = m; l_s[warp] = l; }
+    // the parts' sums in their order, against the largest of their maxima (a part without a tile, or with scores of -inf alone: -inf, weight
+    // 0).  The values of a part of weight 0 are left out, as those of a key of weight 0 are: an infinite one would make a NaN.
+    if (SHARE > 1) __syncthreads();
+    else __syncwarp();
+    if (warp % SHARE) return;
+    float all = m_s[owner][0];
 #pragma unroll
-    for (int i = 0; i < MAXD / 32; ++i) acc_s[warp][lane + 32 * i] = acc[i];
-    __syncthreads();
-    if (part) return;
-    float all = m_s[warp];
-#pragma unroll
-    for (int w = 1; w < SPLIT; ++w) all = fmaxf(all, m_s[warp + w]);
+    for (int w = 1; w < SPLIT; ++w)
+      if (w < used) all = fmaxf(all, m_s[owner][w]);
     l = 0.f;
 #pragma unroll
     for (int i = 0; i < MAXD / 32; ++i) acc[i] = 0.f;
 #pragma unroll
     for (int w = 0; w < SPLIT; ++w) {
-      const float f = gated ? 1.f : expf(m_s[warp + w] - all);
-      l += l_s[warp + w] * f;
+      if (w >= used) break;
+      const float f = gated ? 1.f : expf(m_s[owner][w] - all);
+      l += l_s[owner][w] * f;
       if (f != 0.f)
 #pragma unroll
-        for (int i = 0; i < MAXD / 32; ++i) acc[i] += acc_s[warp + w][lane + 32 * i] * f;
+        for (int i = 0; i < MAXD / 32; ++i) acc[i] += acc_s[owner][w][lane + 32 * i] * f;
     }
   }
   const float inv = gated ? 1.f : 1.f / l;
@@ -255,16 +272,17 @@ LLMK_API int llmk_paged_attention_generic_ex(void* out, long long out_stride, co
   if (window == 0) keep_first = 0;
   const int widest = head_dim > vdim ? head_dim : vdim;
   const long long items = (long long)n_tokens * n_heads;
-  const int per_block = WARPS / split_of(widest);
+  const bool serial = split_of(widest) > 1 && items > (long long)SERIAL_FROM * llmk_sm_count();
+  const int per_block = serial ? WARPS : WARPS / split_of(widest);
   const long long blocks = (items + per_block - 1) / per_block;
   LLMK_REQUIRE(blocks < (1ll << 31), "paged_attention: too many (token, head) items");
   return dispatch_dtype(dtype, [&](auto* tag) {
     using T = LLMK_ELEM(tag);
     const bool vec = head_dim % (16 / (int)sizeof(T)) == 0 && (uintptr_t)k_pages % 16 == 0;      // whole 16-byte pieces per key row
-    auto kern = widest <= 64 ? paged_attention_generic_kernel<T, 64> : widest <= 128 ? paged_attention_generic_kernel<T, 128>
-                : widest <= 256 ? paged_attention_generic_kernel<T, 256>
-                : widest <= 512 ? paged_attention_generic_kernel<T, 512>      // the wide head of a latent attention (its rank)
-                : paged_attention_generic_kernel<T, MAX_HEAD_DIM>;
+    auto kern = serial ? paged_attention_generic_kernel<T, 64, true> : widest <= 64 ? paged_attention_generic_kernel<T, 64, false>
+                : widest <= 128 ? paged_attention_generic_kernel<T, 128, false> : widest <= 256 ? paged_attention_generic_kernel<T, 256, false>
+                : widest <= 512 ? paged_attention_generic_kernel<T, 512, false>      // the wide head of a latent attention (its rank)
+                : paged_attention_generic_kernel<T, MAX_HEAD_DIM, false>;
     launch_kernel(kern, dim3((unsigned)blocks), dim3(WARPS * 32), 0, stream,
         (T*)out, out_stride, (const T*)q, q_stride, (const T*)k_pages, (const T*)v_pages, block_table,
         table_width, token_entry, positions, n_tokens, n_heads, n_kv, head_dim, vdim, page_size, window, keep_first, scale,

@@ -139,3 +139,27 @@ def test_infinite_values_of_keys_that_weigh_nothing(ops, HS):
                                 torch.zeros(1, dtype=torch.int32, device=DEV), torch.tensor([n - 1], dtype=torch.int32, device=DEV), 1, 1, 1, HS, 0, 1.0)
     ref = v[keep].mean(0)
     assert float((out[0].double() - ref).norm() / ref.norm()) < 2e-6
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("HS", [20, 32, 64])
+@pytest.mark.parametrize("window,kw", [(0, {}), (0, dict(sink=True)), (40, dict(keep_first=6)), (0, dict(chunk=150))])
+def test_general_attention_has_the_same_bits_in_launches_of_few_and_many(ops, dtype, HS, window, kw):
+    """Four warps to a head in a launch of few pairs, one warp to a head in a launch of many: the sums are the same ones in the same order."""
+    page, NH, n = 8, 3, 300
+    g = torch.Generator(device=DEV).manual_seed(HS)
+    rand = lambda *s: torch.randn(*s, generator=g, device=DEV).to(dtype)
+    kp, vp, q = rand(-(-n // page), 1, page, HS), rand(-(-n // page), 1, page, HS), rand(n, NH * HS)
+    table = torch.arange(kp.shape[0], dtype=torch.int32, device=DEV)[None].contiguous()
+
+    def run(rows, pos):
+        out = torch.empty(rows.shape[0], NH * HS, device=DEV, dtype=dtype)
+        ops.paged_attention_generic(out, rows.contiguous(), kp, vp, table, torch.zeros(len(pos), dtype=torch.int32, device=DEV), pos, len(pos), NH, 1, HS,
+                                    window, HS ** -0.5, **kw)
+        return out
+
+    at = torch.tensor([0, 31, 32, 63, 64, 95, 96, 127, 128, 299], dtype=torch.int32, device=DEV)
+    few = run(q[at.long()], at)
+    times = 40 * ops.sm_count() // (n * NH) + 1                          # 40 pairs an SM
+    many = run(q.repeat(times, 1), torch.arange(n, dtype=torch.int32, device=DEV).repeat(times)).view(times, n, -1)
+    assert bool((many == many[:1]).all()) and torch.equal(few, many[0][at.long()])
