@@ -2025,7 +2025,7 @@ def gemm_few_available(a, w: torch.Tensor, rows: int) -> bool:
     if not GEMM_FEW or w.dtype != torch.bfloat16 or not gemm_few_takes(rows, w.shape[1]) or w.stride(0) % 8 or w.data_ptr() % 16 or not w.is_cuda:
         return False
     if isinstance(a, NormedRows):
-        return True
+        return a.resid.stride(0) % 4 == 0 and a.resid.data_ptr() % 16 == 0 and a.gain.data_ptr() % 16 == 0
     return a.dtype == torch.bfloat16 and a.is_cuda and a.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0
 
 

@@ -1,0 +1,26 @@
+"""Which products of few rows go to the kernel of their own (gemm_few), on the CPU (operands that only say where they lie)."""
+import types
+
+import pytest
+import torch
+
+
+def weights(n, k):
+    """A bfloat16 matrix on a device, as far as the choice looks at it."""
+    return types.SimpleNamespace(dtype=torch.bfloat16, shape=(n, k), stride=lambda d: (k, 1)[d], data_ptr=lambda: 0, is_cuda=True)
+
+
+def at(offset, *shape):
+    """A float32 tensor whose first number lies `offset` bytes behind a 16-byte boundary."""
+    n = torch.Size(shape).numel()
+    buf = torch.zeros(n + 8)
+    first = (-buf.data_ptr() % 16 + offset) // 4
+    return buf[first:first + n].view(*shape)
+
+
+@pytest.mark.parametrize("resid,gain,want", [(0, 0, True), (0, 4, False), (0, 8, False), (4, 0, False), (8, 8, False)])
+def test_rows_before_their_norm_lie_on_16_bytes(resid, gain, want):
+    """A gain may be a view that a caller gave among the model's tensors: the kernel copies it 16 bytes at a time, the norm's own kernel takes any."""
+    from llm_b200.csrc import ops
+    rows = ops.NormedRows(at(resid, 4, 64), at(gain, 64), 1e-5, 4, torch.bfloat16)
+    assert ops.gemm_few_available(rows, weights(192, 64), 4) == want

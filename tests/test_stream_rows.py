@@ -71,7 +71,8 @@ class Scaled:
         return None
 
 
-def layers(device, tensors):
+def layers(device, tensors, offset=0):
+    """offset: the gains are views that begin so many numbers into a buffer."""
     from llm_b200.models.spec import PartSpec
     from llm_b200.parts.base import part_class, register_part
     from llm_b200.parts.block import PostNormBlock, PreNormBlock, StreamBlock
@@ -90,16 +91,17 @@ def layers(device, tensors):
         for name, info in part.parameters().items():
             g = torch.Generator().manual_seed(len(tensors))
             t = torch.randn(info.shape, generator=g) * (0.12 if info.kind == "matrix" else 0.1)      # sublayers as large as the stream
-            tensors[name] = (t.to(BF16) if info.kind == "matrix" else t + 1.0 if name.endswith("weight") else t).to(device)
+            t = (t.to(BF16) if info.kind == "matrix" else t + 1.0 if name.endswith("weight") else t).to(device)
+            tensors[name] = torch.cat([t[:offset], t])[offset:] if offset and info.shape == (W,) else t
         part.bind(tensors)
     return post, pre, again
 
 
-def check(device, rows, middle):
+def check(device, rows, middle, offset=0):
     """A post-norm layer, then `middle`, then a post-norm layer, against 64 bits."""
     from llm_b200.parts.base import ResidualStream
     tensors = {}
-    post, pre, again = layers(device, tensors)
+    post, pre, again = layers(device, tensors, offset)
     t = {n: v.to(F64) for n, v in tensors.items()}
     rms = lambda x, n: x / torch.sqrt((x * x).mean(-1, keepdim=True) + EPS) * t[n + ".weight"]
     x0 = torch.randn(rows, W, generator=torch.Generator().manual_seed(rows)).to(device)
@@ -136,3 +138,10 @@ def test_rows_after_other_arrangements(rows, middle, monkeypatch):
 @pytest.mark.parametrize("rows", [4, 8, 9, 12])
 def test_rows_after_other_arrangements_on_the_kernels(rows, middle):
     check(torch.device("cuda"), rows, middle)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [4, 9])
+@pytest.mark.parametrize("offset", [1, 2])
+def test_gains_off_the_16_byte_grid(rows, offset):
+    check(torch.device("cuda"), rows, "prenorm", offset)
