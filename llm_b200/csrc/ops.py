@@ -2053,6 +2053,11 @@ def gemm_few(a, w: torch.Tensor, out: torch.Tensor, rows: int, kind=None, bias=N
     return out
 
 
+def gemm_few_sums_fit(rows: int, n: int) -> bool:
+    """Whether the scratch buffer of unsummed products holds so many results."""
+    return rows * n * 4 <= _PARTIAL_BYTES
+
+
 def gemm_few_sums(a, w: torch.Tensor, rows: int, dtype: torch.dtype) -> PartialSum:
     """a[:rows] @ w.T as a PartialSum of one term: float32 sums for a kernel that takes one, with nothing rounded in between."""
     part = _partials(w.device)

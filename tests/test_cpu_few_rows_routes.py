@@ -24,3 +24,17 @@ def test_rows_before_their_norm_lie_on_16_bytes(resid, gain, want):
     from llm_b200.csrc import ops
     rows = ops.NormedRows(at(resid, 4, 64), at(gain, 64), 1e-5, 4, torch.bfloat16)
     assert ops.gemm_few_available(rows, weights(192, 64), 4) == want
+
+
+@pytest.mark.parametrize("rows,n,unsummed", [(8, 1 << 21, True), (8, (1 << 21) + 8, False), (1, 1 << 24, True), (1, (1 << 24) + 8, False)])
+def test_results_beyond_the_scratch_buffer_are_written_out(rows, n, unsummed, monkeypatch):
+    """64 MB of float32 sums are what the buffer holds."""
+    from llm_b200.csrc import ops
+    from llm_b200.parts.linear import linear
+    out = types.SimpleNamespace(dtype=torch.bfloat16, shape=(rows, n))
+    monkeypatch.setattr(ops, "gemm_few_available", lambda a, w, rows: True)
+    monkeypatch.setattr(ops, "gemm_few", lambda a, w, out, rows, **k: out)
+    monkeypatch.setattr(ops, "_partials", lambda device: torch.empty(ops._PARTIAL_BYTES // 4, device="meta"))
+    w = types.SimpleNamespace(shape=(n, 64), device="meta")
+    got = linear(None, w, out, rows, allow_partial=True)
+    assert isinstance(got, ops.PartialSum) if unsummed else got is out
