@@ -14,6 +14,7 @@
 //
 // Tiles hold as many rows as divide the weight rows evenly over the SMs (14 of the 16 for 2,048 rows on 148 SMs); a CTA walks over its
 // tiles with the stream running across them.
+#include <atomic>
 #include <mutex>
 
 #include "tcgen05.cuh"
@@ -366,20 +367,6 @@ int encode_weights(CUtensorMap* out, const void* w, long long rows, int K, long 
   return r == CUDA_SUCCESS ? 0 : llmk_fail(-2, "cuTensorMapEncodeTiled failed with %d", (int)r);
 }
 
-template <bool KEEP>
-int launch_few(const CUtensorMap& map, const CUtensorMap& tail, const FewArgs& p, int out_kind, int grid, size_t smem, cudaStream_t stream) {
-  void (*kern)(CUtensorMap, CUtensorMap, FewArgs) =
-      out_kind == FEW_OUT_F32 ? few_rows_kernel<FEW_OUT_F32, KEEP> : out_kind == FEW_OUT_BF16 ? few_rows_kernel<FEW_OUT_BF16, KEEP>
-      : out_kind == FEW_OUT_ADD ? few_rows_kernel<FEW_OUT_ADD, KEEP> : out_kind == FEW_OUT_SILU ? few_rows_kernel<FEW_OUT_SILU, KEEP>
-      : out_kind == FEW_OUT_RELU ? few_rows_kernel<FEW_OUT_RELU, KEEP> : few_rows_kernel<FEW_OUT_CLAMPED, KEEP>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return llmk_fail((int)e, "gemm_few: %s", cudaGetErrorString(e));
-  }
-  launch_kernel(kern, dim3(grid), dim3(FEW_WARPS * 32 + 32), smem, stream, map, tail, p);
-  LLMK_LAUNCH_CHECK("gemm_few");
-}
-
 // What must be left beside the rows, in boxes: 8 rows of 8,448 leave room for three, and the tcgen05 kernel's swapped mode is ahead then (a call of the
 // design with that width 21.50 ms against 21.58); 3 rows of 14,336 leave four, and a decode step takes 3,198 us against 3,253.
 constexpr int FEW_SMEM = 227 * 1024, FEW_LEAST_STAGES = 4;
@@ -387,6 +374,26 @@ constexpr int FEW_SMEM = 227 * 1024, FEW_LEAST_STAGES = 4;
 // ring first: 64 KB 771, 795, 828 us; 100 KB 695, 712, 746; 140 KB 666, 690, 750; 200 KB 677, 719, 755 (649, 675, 738 with 140 KB once the rows
 // were kept in registers); of 140 KB first 96 KB: 634, 665, 717; 72 KB: 629, 667, 716; 57 KB: 638, 668, 727.
 constexpr int FEW_RING = 140 * 1000, FEW_EARLY = 72 * 1000;
+
+template <bool KEEP>
+int launch_few(const CUtensorMap& map, const CUtensorMap& tail, const FewArgs& p, int out_kind, int grid, size_t smem, cudaStream_t stream) {
+  void (*kern)(CUtensorMap, CUtensorMap, FewArgs) =
+      out_kind == FEW_OUT_F32 ? few_rows_kernel<FEW_OUT_F32, KEEP> : out_kind == FEW_OUT_BF16 ? few_rows_kernel<FEW_OUT_BF16, KEEP>
+      : out_kind == FEW_OUT_ADD ? few_rows_kernel<FEW_OUT_ADD, KEEP> : out_kind == FEW_OUT_SILU ? few_rows_kernel<FEW_OUT_SILU, KEEP>
+      : out_kind == FEW_OUT_RELU ? few_rows_kernel<FEW_OUT_RELU, KEEP> : few_rows_kernel<FEW_OUT_CLAMPED, KEEP>;
+  // once per build and device, the most that any launch asks for: the size belongs to the kernel and not to the launch, and another thread's
+  // smaller one, set between this thread's setting and its launch, would make the launch fail
+  static std::atomic<bool> ready[FEW_OUT_CLAMPED + 1][64];
+  int device = -1;
+  const bool known = cudaGetDevice(&device) == cudaSuccess && device >= 0 && device < 64;
+  if (!known || !ready[out_kind][device].load(std::memory_order_acquire)) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_SMEM);
+    if (e != cudaSuccess) return llmk_fail((int)e, "gemm_few: %s", cudaGetErrorString(e));
+    if (known) ready[out_kind][device].store(true, std::memory_order_release);
+  }
+  launch_kernel(kern, dim3(grid), dim3(FEW_WARPS * 32 + 32), smem, stream, map, tail, p);
+  LLMK_LAUNCH_CHECK("gemm_few");
+}
 
 }  // namespace
 

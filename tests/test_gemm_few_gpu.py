@@ -107,3 +107,26 @@ def test_what_is_not_taken(ops):
     for rows in range(0, 18):
         for k in (64, 96, 2048, 4096, 5632, 14336, 16384, 65536):
             assert bool(ops.load_tensor().llmk_gemm_few_supported(rows, k)) == ops.gemm_few_takes(rows, k), (rows, k)
+
+
+def test_two_threads_with_products_of_different_sizes(ops):
+    """Each launch takes the shared memory that its rows and stages need, whatever another thread launches at the same time."""
+    import threading
+    small, large = operands(1, 96, 64), operands(8, 2368, 5632)
+    want = [ops.gemm_few(a, w, torch.empty(a.shape[0], w.shape[0], device=DEV), a.shape[0]) for a, w in (small, large)]
+    outs, errors = [torch.empty_like(t) for t in want], []
+
+    def loop(a, w, out):
+        try:
+            for _ in range(3000):
+                ops.gemm_few(a, w, out, a.shape[0])
+        except Exception as e:      # noqa: BLE001
+            errors.append(e)
+
+    threads = [threading.Thread(target=loop, args=(a, w, o)) for (a, w), o in zip((small, large), outs)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors and all(torch.equal(o, t) for o, t in zip(outs, want))
