@@ -75,7 +75,7 @@ struct FewArgs {
   int tiles, stages, boxes;    // boxes: of a step
   const float* bias;           // of the weight rows, or null
   float limit, alpha;          // of the clamped unit
-  int early;                   // steps that are asked for before the rows
+  int early;                   // steps that are asked for before the rows, at most the stages
   int* error;
 };
 
@@ -121,7 +121,8 @@ few_rows_kernel(const __grid_constant__ CUtensorMap weights, const __grid_consta
       const int n = min(tile * p.tile, p.N - p.tile);  // the last tile ends with the weights, and repeats rows of the one before
       for (int b = 0; b < all_boxes;) {
         // what a load waits for is what was asked for before it: the rows come before all but the first steps
-        if (issued == p.early) ok = tc::mbar_wait(asked, 0);
+        // (and the bounded waits, from this one on, begin when the kernels before this one have ended, however long they take)
+        if (issued == p.early) { pdl_wait(); ok = tc::mbar_wait(asked, 0); }
         ok = ok && tc::mbar_wait(empty + s, phase);
         if (!ok) break;
         const int end = min(b + p.boxes, all_boxes);
@@ -436,6 +437,7 @@ LLMK_API int llmk_gemm_few(const void* a, const float* x, const float* gain, flo
   if (p.stages > FEW_MAX_STAGES) p.stages = FEW_MAX_STAGES;
   p.early = FEW_EARLY / (p.boxes * box_bytes);
   if (p.early < 1) p.early = 1;
+  if (p.early > p.stages) p.early = p.stages;      // no stage is waited for before the rows
   // at least half of the shared memory: a CTA that shared its SM with another of the same launch would end long after the rest (a kernel that
   // starts while the one before it leaves SMs finds room for two on some: a decode step of 1.1 B then took 880 us instead of 720)
   const size_t need = rest + (size_t)p.stages * p.boxes * box_bytes, smem = need < FEW_SMEM / 2 + 1024 ? FEW_SMEM / 2 + 1024 : need;

@@ -130,3 +130,20 @@ def test_two_threads_with_products_of_different_sizes(ops):
         t.join()
     torch.cuda.synchronize()
     assert not errors and all(torch.equal(o, t) for o, t in zip(outs, want))
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 148, 2048), (8, 2368, 5632), (8, 148, 8192 - 64)])
+def test_behind_a_kernel_that_takes_longer_than_the_waits(ops, M, N, K):
+    """The kernel starts under the one before it and asks for weights; its bounded waits (2e9 cycles, a second) count from that one's end."""
+    a, w = operands(M, N, K)
+    want = ops.gemm_few(a, w, torch.empty(M, N, device=DEV), M)
+    x, y = torch.ones(1, 40_000_001, device=DEV), torch.ones(1, 40_000_001, device=DEV)      # one tile, a long chain of k
+    one, out = torch.empty(1, 1, device=DEV), torch.empty(M, N, device=DEV)
+    begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    begin.record()
+    ops.gemm_simt(x, y, one, 1)
+    ops.gemm_few(a, w, out, M)
+    end.record()
+    torch.cuda.synchronize()
+    assert begin.elapsed_time(end) > 1200
+    assert ops.gemm_tc_take_error() == 0 and torch.equal(out, want)
