@@ -31,7 +31,7 @@ import math
 import torch
 
 from ..csrc import ops
-from .base import CacheNeed, ParamInfo, Part, StateNeed, build_part, register_part
+from .base import CacheNeed, ParamInfo, Part, StateNeed, build_part, register_part, takes
 from .linear import FUSE_PARTIALS, linear, linear_add
 
 
@@ -195,6 +195,7 @@ class PagedAttention(Part):
     def reads_unformed(self, rows, ctx) -> bool:
         return not self.extended and ops.gemm_few_available(rows, self.w_qkv, ctx.n_tokens)
 
+    @takes("into", "whole")
     def forward(self, x: torch.Tensor, ctx, view, into=None, whole: bool = False):
         """into: the stream that a last product of few rows may add to (the result is then None); whole: no unsummed result."""
         T = ctx.n_tokens

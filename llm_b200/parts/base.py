@@ -11,7 +11,8 @@ Roles and what each must provide, beyond Part:
   norm       forward(stream, ctx) -> rows [T, H] in the compute dtype; folds the
              stream's pending term into the residual first.
   mixer      cache_need() / state_need(); forward(x, ctx, view) -> [T, H].
-  ffn        forward(x, ctx) -> [T, H].
+  ffn        forward(x, ctx) -> [T, H].  (Mixers and feed-forwards whose forward is marked with `takes` may be given more,
+             and return None.)
   position   either tables() -> (cos, sin) float32 [max_position, head_dim/2] for the kernels that
              rotate half a head against the other (fused with the cache store), or apply(q, k,
              ctx): its own in-place transform of the step's queries [T, heads, head_dim] and new
@@ -117,6 +118,25 @@ class Part:
         """Whether this step's launches of the part depend only on the step's numbers of entries,
         tokens and wanted rows (and the key bucket), so that a captured graph may be replayed."""
         return True
+
+
+def takes(*options: str):
+    """Marks a mixer's or feed-forward's `forward` as one that takes these options of the arrangement that calls it:
+
+      into    the residual stream, to which the part may add its result itself (linear_add); it then returns None
+      whole   True: the result is a tensor, not one that is still to be summed (ops.PartialSum)
+
+    A part whose forward takes `into` may also have reads_unformed(rows, ctx): whether, in this step, it reads rows before
+    their norm (ops.NormedRows) in place of the tensor.  The mark belongs to the function: a subclass with a forward of its own
+    is called without them unless it is marked too."""
+    def mark(forward):
+        forward.takes_options = frozenset(options)
+        return forward
+    return mark
+
+
+def takes_option(part, option: str) -> bool:
+    return part is not None and option in getattr(type(part).forward, "takes_options", ())
 
 
 _REGISTRIES: Dict[str, Dict[str, Callable]] = {

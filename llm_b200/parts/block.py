@@ -8,11 +8,10 @@ out norm2 and ffn: it is x += mixer(norm1(x)) alone.
 from __future__ import annotations
 
 import dataclasses
-import inspect
 
 import torch
 
-from .base import ResidualStream, StateNeed, build_part, register_part
+from .base import ResidualStream, StateNeed, build_part, register_part, takes_option
 
 
 class PreNormBlock:
@@ -29,8 +28,7 @@ class PreNormBlock:
         self.norm1, self.mixer = self.parts["norm1"], self.parts["mixer"]
         self.norm2, self.ffn = self.parts["norm2"], self.parts["ffn"]
         # a part whose forward takes `into` may read rows before their norm and add its result to the stream itself
-        takes = lambda part: part is not None and "into" in inspect.signature(part.forward).parameters
-        self.mixer_into, self.ffn_into = takes(self.mixer), takes(self.ffn)
+        self.mixer_into, self.ffn_into = takes_option(self.mixer, "into"), takes_option(self.ffn, "into")
         # a feed-forward that keeps something per request (the inputs of a convolution over time) says so with state_need();
         # the layer's state row is then the mixer's numbers followed by the feed-forward's
         self.ffn_state = self.ffn.state_need() if self.ffn is not None and hasattr(self.ffn, "state_need") else None

@@ -21,7 +21,7 @@ import math
 import torch
 
 from ..csrc import ops
-from .base import CacheNeed, ParamInfo, Part, register_part
+from .base import CacheNeed, ParamInfo, Part, register_part, takes
 from .linear import FUSE_PARTIALS, linear, linear_add
 
 _NAMES = {"q": "q", "k": "k", "v": "v", "gate": "g", "out": "o", "q_norm": "q.norm", "k_norm": "k.norm",
@@ -78,6 +78,7 @@ class DifferentialAttention(Part):
     def state_need(self):
         return None
 
+    @takes("into")
     def forward(self, x: torch.Tensor, ctx, view, into=None):
         T, ws = ctx.n_tokens, ctx.workspace
         H, G, D, V = self.num_heads, self.num_kv_heads, self.head_dim, self.value_dim

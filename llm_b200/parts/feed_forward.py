@@ -10,7 +10,7 @@ from __future__ import annotations
 import torch
 
 from ..csrc import ops
-from .base import ParamInfo, Part, register_part
+from .base import ParamInfo, Part, register_part, takes
 from .linear import FUSE_PARTIALS, linear, linear_act, linear_add, linear_swiglu
 
 
@@ -61,6 +61,7 @@ class SwiGLU(Part):
     def reads_unformed(self, rows, ctx) -> bool:
         return ops.gemm_few_available(rows, self.w_gate_up, ctx.n_tokens)
 
+    @takes("into")
     def forward(self, x: torch.Tensor, ctx, tag: str = "ffn", into=None):
         T, ws = ctx.n_tokens, ctx.workspace
         act = ws.get(tag + "_act", T, self.intermediate_size, self.dtype)
@@ -114,6 +115,7 @@ class ActMLP(Part):
             self.b_up = tensors[self.name(self.up_name + ".b")].contiguous()
             self.b_down = tensors[self.name(self.down_name + ".b")].contiguous()
 
+    @takes("into")
     def forward(self, x: torch.Tensor, ctx, tag: str = "ffn", allow_unsummed: bool = False, into=None):
         T, ws = ctx.n_tokens, ctx.workspace
         act = ws.get(tag + "_act", T, self.intermediate_size, self.dtype)

@@ -32,7 +32,7 @@ from __future__ import annotations
 import torch
 
 from ..csrc import ops
-from .base import CacheNeed, ParamInfo, Part, build_part, register_part
+from .base import CacheNeed, ParamInfo, Part, build_part, register_part, takes
 from .linear import FUSE_PARTIALS, linear, linear_add
 
 _NAMES = {"q": "q", "down": "dkv", "down_norm": "dkv.norm", "up_k": "uk", "up_v": "uv", "gate": "g", "out": "o",
@@ -214,6 +214,7 @@ class LatentAttention(Part):
             return None
         return linear(attn, self.w_o, ws.get("mixer_out", T, self.hidden_size, self.dtype), T, allow_partial=FUSE_PARTIALS)
 
+    @takes("into")
     def forward(self, x: torch.Tensor, ctx, view, into=None):
         if self.rotary:
             return self._forward_rotary(x, ctx, view, into)

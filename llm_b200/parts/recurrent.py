@@ -21,12 +21,11 @@ step sizes, states and the norms are float32; projections and convolutions run i
 from __future__ import annotations
 
 import dataclasses
-import inspect
 
 import torch
 
 from ..csrc import ops
-from .base import ParamInfo, Part, StateNeed, build_part, register_part
+from .base import ParamInfo, Part, StateNeed, build_part, register_part, takes_option
 from .linear import FUSE_PARTIALS, linear
 
 
@@ -480,7 +479,7 @@ class ParallelMixers(Part):
         self.hidden_size, self.eps = int(hidden_size), float(eps)
         self.left_name, self.right_name = left_name, right_name
         self.left, self.right = build_part("mixer", left, dtype, device), build_part("mixer", right, dtype, device)
-        self.left_whole = "whole" in inspect.signature(self.left.forward).parameters
+        self.left_whole = takes_option(self.left, "whole")
         if self.left.cache_need() is not None and self.right.cache_need() is not None:
             raise ValueError("parallel mixers: only one side may keep keys and values")
         self.left_cols = _pad4(_state_numel(self.left.state_need()))
