@@ -168,6 +168,10 @@ hc_norm_vec_kernel(float* __restrict__ resid, MaybePartial<T> y, const float* __
 // token is bound by one SM's way to L2 (64 KB both ways at four streams of 2,048) and by 160 multiply-adds a thread.  Float32 rows,
 // whose sums do not depend on how many rows there are, never come here.  8 rows inside decode steps: 7.3 -> 2.6 us a launch; the norm of one stream
 // over the unsummed terms of a product (add_rmsnorm, 64 rows) gained nothing this way (3.4, 3.6 us).
+// Where it is taken: while a CTA has an SM to itself, from two streams on (launches one behind another, one CTA a token / a cluster, 2 streams of
+// 2,048: 8 rows 2.69 / 2.40 us, 37 rows 2.69 / 2.66, 64 rows 2.88 / 3.04, 74 rows 2.72 / 3.24; 4 streams of 1,536: 8 rows 2.89 / 2.49, 74 rows 2.91 /
+// 3.26; one stream 2.29 / 2.49), and up to two CTAs an SM for rows of 32 KB, which keep one CTA longer (4 streams of 2,048: 8 rows 3.30 / 2.48, 64
+// rows 3.70 / 3.40, 74 rows 3.39 / 3.36).  Widths: two columns a thread of 256 at most, which end at 2,048; up to 512 both took the same, 2.1 us.
 constexpr int HC_CTAS = 4;
 
 template <int S>
@@ -279,8 +283,9 @@ LLMK_API int llmk_hc_norm(float* resid, const void* y, const float* partials, in
     const bool vec = hidden % 8 == 0 && (uintptr_t)resid % 16 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)partials % 16 == 0 &&
                      split_stride % 4 == 0 && (uintptr_t)out % 16 == 0;
     if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-      if (vec && n_tokens * HC_CTAS <= 2 * llmk_sm_count() && streams <= 4 && hidden >= 1024 && hidden <= HC_CTAS * 256 * 2) {
-        auto kern = streams == 1 ? hc_norm_cluster_kernel<1> : streams == 2 ? hc_norm_cluster_kernel<2> : streams == 3 ? hc_norm_cluster_kernel<3>
+      const int most = (streams * hidden >= 8192 ? 2 : 1) * llmk_sm_count();      // CTAs (see HC_CTAS)
+      if (vec && n_tokens * HC_CTAS <= most && streams >= 2 && streams <= 4 && hidden >= 1024 && hidden <= HC_CTAS * 256 * 2) {
+        auto kern = streams == 2 ? hc_norm_cluster_kernel<2> : streams == 3 ? hc_norm_cluster_kernel<3>
                                                                                                         : hc_norm_cluster_kernel<4>;
         const int threads = ((hidden + HC_CTAS * 2 - 1) / (HC_CTAS * 2) + 31) / 32 * 32;
         launch_clusters(kern, dim3(n_tokens * HC_CTAS), dim3(threads), HC_CTAS, stream, resid, yy, write_mix, write_out, read_in, gain, (T*)out, hidden,

@@ -16,7 +16,7 @@ def partials(ops, y, splits):
 
 
 @pytest.mark.parametrize("streams,hidden", [(1, 1024), (2, 1032), (3, 2040), (4, 2048), (4, 2056), (5, 1024)])
-@pytest.mark.parametrize("rows", [1, 8, 74, 75])
+@pytest.mark.parametrize("rows", [1, 8, 37, 38, 74, 75])
 @pytest.mark.parametrize("splits", [None, 0, 1, 5])
 def test_hc_norm(rows, streams, hidden, splits):
     from llm_b200.csrc import ops
