@@ -175,7 +175,7 @@ class ClampedGLU(Part):
         T, ws = ctx.n_tokens, ctx.workspace
         I = self.intermediate_size
         act = ws.get("ffn_act", T, I, self.dtype)
-        if T and ops.gemm_few_available(x, self.w_gate_up, T):      # few rows: the unit in the product's epilogue
+        if T and ops.gemm_few_available(x, self.w_gate_up, T, gated=True):      # few rows: the unit in the product's epilogue
             ops.gemm_few(x, self.w_gate_up, act, T, kind="clamped", bias=self.b_gate_up, limit=self.limit, alpha=self.alpha)
         else:
             # one product for gate and up; its split-K partial results go unsummed to the activation kernel, which

@@ -66,7 +66,7 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, rows
     kernel."""
     if rows == 0:
         return True
-    if act in ("silu", "relu") and ops.gemm_few_available(x, weight, rows):
+    if act in ("silu", "relu") and ops.gemm_few_available(x, weight, rows, gated=True):
         ops.gemm_few(x, weight, out, rows, kind=act)
         return True
     if x.dtype != torch.bfloat16 or not ops.gemm_swiglu_available(x, weight, out, rows):

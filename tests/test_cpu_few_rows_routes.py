@@ -19,9 +19,10 @@ def at(offset, *shape):
 
 
 @pytest.mark.parametrize("resid,gain,want", [(0, 0, True), (0, 4, False), (0, 8, False), (4, 0, False), (8, 8, False)])
-def test_rows_before_their_norm_lie_on_16_bytes(resid, gain, want):
+def test_rows_before_their_norm_lie_on_16_bytes(resid, gain, want, monkeypatch):
     """A gain may be a view that a caller gave among the model's tensors: the kernel copies it 16 bytes at a time, the norm's own kernel takes any."""
     from llm_b200.csrc import ops
+    monkeypatch.setattr(ops, "sm_count", lambda: 148)
     rows = ops.NormedRows(at(resid, 4, 64), at(gain, 64), 1e-5, 4, torch.bfloat16)
     assert ops.gemm_few_available(rows, weights(192, 64), 4) == want
 
@@ -38,3 +39,17 @@ def test_results_beyond_the_scratch_buffer_are_written_out(rows, n, unsummed, mo
     w = types.SimpleNamespace(shape=(n, 64), device="meta")
     got = linear(None, w, out, rows, allow_partial=True)
     assert isinstance(got, ops.PartialSum) if unsummed else got is out
+
+
+@pytest.mark.parametrize("n,k,plain,fused", [(2368, 64, True, True), (2369, 64, False, True), (11840, 64, False, True), (11841, 64, False, False),
+                                             (4736, 256, True, True), (4737, 256, False, True), (11840, 512, True, True), (21312, 512, False, True),
+                                             (21313, 512, False, False), (32000, 512, False, False), (32000, 768, False, True), (32000, 1024, True, True),
+                                             (128256, 1024, True, True), (128256, 4096, True, True)])
+def test_short_rows_on_many_tiles_take_the_other_kernel(n, k, plain, fused, monkeypatch):
+    from llm_b200.csrc import ops
+    monkeypatch.setattr(ops, "sm_count", lambda: 148)
+    rows = torch.zeros(4, k, dtype=torch.bfloat16)
+    a = types.SimpleNamespace(dtype=torch.bfloat16, is_cuda=True, stride=rows.stride, data_ptr=lambda: 0)
+    normed = ops.NormedRows(at(0, 4, k), at(0, k), 1e-5, 4, torch.bfloat16)
+    assert ops.gemm_few_available(a, weights(n, k), 4) == plain
+    assert ops.gemm_few_available(a, weights(n, k), 4, gated=True) == ops.gemm_few_available(normed, weights(n, k), 4) == fused

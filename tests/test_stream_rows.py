@@ -51,7 +51,7 @@ def plain_kernels(monkeypatch):
 
     put("add_rmsnorm", add_rmsnorm), put("sum_rmsnorm", sum_rmsnorm), put("add_layernorm", add_layernorm), put("gemm_few", gemm_few)
     put("silu_mul", silu_mul), put("concat_embedding", concat_embedding)
-    put("gemm_few_available", lambda a, w, rows: rows <= 8)
+    put("gemm_few_available", lambda a, w, rows, gated=False: rows <= 8)
     put("gemm_few_sums", lambda a, w, rows, dtype: gemm_few(a, w, torch.empty(rows, w.shape[0], dtype=dtype), rows))
     put("gemm_simt", lambda a, w, out, rows: out[:rows].copy_(a[:rows].float() @ w.float().T))
     put("add_bias", lambda x, bias, rows: x[:rows].add_(bias.to(x.dtype)))
