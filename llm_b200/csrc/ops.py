@@ -2073,6 +2073,14 @@ def gemm_few_sums_fit(rows: int, n: int) -> bool:
     return rows * n * 4 <= _PARTIAL_BYTES
 
 
+def gemm_few_sums_pay(a, rows: int) -> bool:
+    """Whether the few-row product is the faster one where the kernel behind it takes sums of several terms: every CTA reads all of the rows, and
+    from 64 KB of them on the tcgen05 kernel, which splits K over CTAs, is as fast or faster when nothing else has to sum its terms.  Replayed
+    decode steps with it / with this one: 6 rows of 8,448 575.3 / 580.4 us, 8 rows of 5,632 573.6 / 577.6, 4 rows of 8,448 559.4 / 561.8, 8 rows of
+    4,096 3,018 / 3,025, 6 rows of 5,632 567.0 / 567.8; below, 4 rows of 5,632 566.0 / 562.4, 8 rows of 2,048 519 / 503."""
+    return isinstance(a, NormedRows) or rows * a.shape[1] < 32768
+
+
 def gemm_few_sums(a, w: torch.Tensor, rows: int, dtype: torch.dtype) -> PartialSum:
     """a[:rows] @ w.T as a PartialSum of one term: float32 sums for a kernel that takes one, with nothing rounded in between."""
     part = _partials(w.device)

@@ -36,7 +36,10 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, rows: int, 
         allow_partial = False
     if ops.gemm_few_available(x, weight, rows):      # a bias joins the sums
         sums = allow_partial and out.dtype != torch.float32 and ops.gemm_few_sums_fit(rows, weight.shape[0])
-        return ops.gemm_few_sums(x, weight, rows, out.dtype) if sums else ops.gemm_few(x, weight, out, rows, bias=bias)
+        if not sums:
+            return ops.gemm_few(x, weight, out, rows, bias=bias)
+        if ops.gemm_few_sums_pay(x, rows):
+            return ops.gemm_few_sums(x, weight, rows, out.dtype)
     if x.dtype == torch.bfloat16 and ops.gemm_fast_available(x, weight, out, rows):
         res = ops.gemm_fast(x, weight, out, rows, allow_partial=allow_partial, cta_limit=cta_limit)
     else:

@@ -35,6 +35,7 @@ def test_results_beyond_the_scratch_buffer_are_written_out(rows, n, unsummed, mo
     out = types.SimpleNamespace(dtype=torch.bfloat16, shape=(rows, n))
     monkeypatch.setattr(ops, "gemm_few_available", lambda a, w, rows: True)
     monkeypatch.setattr(ops, "gemm_few", lambda a, w, out, rows, **k: out)
+    monkeypatch.setattr(ops, "gemm_few_sums_pay", lambda a, rows: True)
     monkeypatch.setattr(ops, "_partials", lambda device: torch.empty(ops._PARTIAL_BYTES // 4, device="meta"))
     w = types.SimpleNamespace(shape=(n, 64), device="meta")
     got = linear(None, w, out, rows, allow_partial=True)
@@ -53,3 +54,23 @@ def test_short_rows_on_many_tiles_take_the_other_kernel(n, k, plain, fused, monk
     normed = ops.NormedRows(at(0, 4, k), at(0, k), 1e-5, 4, torch.bfloat16)
     assert ops.gemm_few_available(a, weights(n, k), 4) == plain
     assert ops.gemm_few_available(a, weights(n, k), 4, gated=True) == ops.gemm_few_available(normed, weights(n, k), 4) == fused
+
+
+@pytest.mark.parametrize("rows,k,want", [(8, 4032, "few"), (8, 4096, "split"), (5, 6528, "few"), (5, 6592, "split"), (1, 14336, "few")])
+@pytest.mark.parametrize("kind", ["unsummed", "whole", "biased", "normed"])
+def test_unsummed_products_of_long_rows_are_split(rows, k, want, kind, monkeypatch):
+    """Only where the next kernel takes several terms, and the rows are there as they are multiplied."""
+    from llm_b200.csrc import ops
+    from llm_b200.parts.linear import linear
+    sent = []
+    monkeypatch.setattr(ops, "gemm_few_available", lambda a, w, rows: True)
+    monkeypatch.setattr(ops, "gemm_fast_available", lambda *a: True)
+    monkeypatch.setattr(ops, "gemm_fast", lambda *a, **k: sent.append("split"))
+    monkeypatch.setattr(ops, "gemm_few", lambda *a, **k: sent.append("few"))
+    monkeypatch.setattr(ops, "gemm_few_sums", lambda *a, **k: sent.append("few"))
+    x = torch.zeros(rows, k, dtype=torch.bfloat16)
+    if kind == "normed":
+        x = ops.NormedRows(x.float(), torch.zeros(k), 1e-5, rows, torch.bfloat16)
+    linear(x, torch.zeros(96, k, dtype=torch.bfloat16), torch.zeros(rows, 96, dtype=torch.bfloat16), rows, allow_partial=kind != "whole",
+           bias=torch.zeros(96) if kind == "biased" else None)
+    assert sent == [want if kind == "unsummed" else "few"]
