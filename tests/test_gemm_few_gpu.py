@@ -21,12 +21,17 @@ def operands(M, N, K, seed=0):
 
 # K: one block, a box and a ragged one, several steps with a ragged last; N: fewer than SMs, no multiple of a tile, several tiles a CTA
 SIZES = [(96, 64), (17, 512), (2369, 576), (300, 1408), (2560, 2048), (5000, 2624)]
-# float32 sums of K terms in blocks: (K / 64 + 64) roundings of 2^-24 at most on the largest partial sum, as a share of the terms' norm
-BOUND = 2e-6
+# more passes of the loops that stage the rows (64 blocks of 64 a pass), the second one ragged, whole, and up to four; few outputs, to keep it quick
+LONG = [(1, 300, 4160), (3, 300, 4160), (1, 100, 5632), (8, 100, 5632), (1, 64, 14336), (3, 64, 14336)]
 
 
-@pytest.mark.parametrize("M", [1, 3, 7, 8])
-@pytest.mark.parametrize("N,K", SIZES)
+def bound(K):
+    """Of the distance from the exact sum, as a share of the sum of the terms' absolute values: an accumulator takes 2 MMAs of each of its warp's blocks, a
+    block of 64 k in every 512, and each may cut off 2^-23 of what it has; two accumulators, eight warps and the factor behind them: ten roundings."""
+    return (2 * -(-K // 512) + 10) * 2.0 ** -23
+
+
+@pytest.mark.parametrize("M,N,K", [(m, n, k) for m in (1, 3, 7, 8) for n, k in SIZES] + LONG)
 def test_sums(ops, M, N, K):
     a, w = operands(M, N, K)
     assert ops.gemm_few_available(a, w, M)
@@ -34,7 +39,7 @@ def test_sums(ops, M, N, K):
     scale = (a.double().abs() @ w.double().abs().T)
     out = torch.full((M + 1, N + 3), 7.0, device=DEV)
     ops.gemm_few(a, w, out[:, :N], M)
-    assert bool(((out[:M, :N].double() - exact).abs() <= BOUND * scale + 1e-30).all())
+    assert bool(((out[:M, :N].double() - exact).abs() <= bound(K) * scale + 1e-30).all())
     assert bool((out[M] == 7).all()) and bool((out[:, N:] == 7).all())            # nothing beside the results
     half = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
     ops.gemm_few(a, w, half, M)
@@ -57,12 +62,16 @@ def test_gated(ops, M, N, K, act):
     out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
     ops.gemm_few(a, w, out, M, kind=act)
     # one rounding of the result, and the sums' errors through a product whose factors have slopes of at most 1.1
-    slack = 2.0 ** -8 * ref.abs() + 1.2 * BOUND * (scale[:, :N] * u.abs() + scale[:, N:] * g.abs()) + 1e-12
+    slack = 2.0 ** -8 * ref.abs() + 1.2 * bound(K) * (scale[:, :N] * u.abs() + scale[:, N:] * g.abs()) + 1e-12
     assert bool(((out.double() - ref).abs() <= slack).all())
 
 
-@pytest.mark.parametrize("M", [1, 2, 8])
-@pytest.mark.parametrize("N,K", [(40, 64), (300, 1408), (2560, 2048)])
+# under a norm a pass takes 32 blocks: K of one pass, of a second one of one block, of two whole ones, of a third; the last: a stage of a single box beside
+# the rows, tiles of 16
+NORMED = [(m, n, k) for m in (1, 2, 8) for n, k in ((40, 64), (300, 1408), (2560, 2048), (200, 2112), (96, 4096), (40, 4160))] + [(8, 2368, 7168)]
+
+
+@pytest.mark.parametrize("M,N,K", NORMED)
 def test_rows_under_a_norm(ops, M, N, K):
     _, w = operands(M, N, K)
     x = torch.randn(M + 2, K, device=DEV) * torch.tensor([0.01, 300.0] * (M + 2), device=DEV)[:M + 2, None]
@@ -74,6 +83,32 @@ def test_rows_under_a_norm(ops, M, N, K):
     # one rounding to bfloat16 (2^-9 of each) of what multiplies the weights, the rest in float32
     scale = h.abs() @ w.double().abs().T
     assert bool(((out.double() - h @ w.double().T).abs() <= (2.0 ** -9 + 1e-5) * scale).all())
+
+
+@pytest.mark.parametrize("M", [1, 5, 8])
+@pytest.mark.parametrize("N,K", [(34, 64), (300, 2048), (200, 2112), (1190, 4096), (40, 4160)])
+@pytest.mark.parametrize("act", ["silu", "relu", "clamped"])
+def test_gated_on_rows_under_a_norm(ops, M, N, K, act):
+    """The form of a decode step's feed-forward: the norm before the product and the activation behind it."""
+    _, w = operands(M, 2 * N, K)
+    x = torch.randn(M, K, device=DEV) * torch.tensor([0.01, 300.0, 1.0] * M, device=DEV)[:M, None]
+    gain = 1.0 + 0.1 * torch.randn(K, device=DEV)
+    bias = torch.randn(2 * N, device=DEV) if act == "clamped" else None
+    out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    ops.gemm_few(ops.NormedRows(x, gain, 1e-5, M, torch.bfloat16), w, out, M, kind=act, bias=bias, limit=1.5, alpha=1.702)
+    xd = x.double()
+    h = xd / torch.sqrt((xd * xd).mean(-1, keepdim=True) + 1e-5) * gain.double()
+    z = h @ w.double().T + (bias.double() if bias is not None else 0)
+    err = (2.0 ** -9 + 1e-5) * (h.abs() @ w.double().abs().T)           # of the two sums: what multiplies the weights is rounded once to bfloat16
+    (g, u), (eg, eu) = z.chunk(2, -1), err.chunk(2, -1)
+    if act == "clamped":
+        g, u = g.clamp(max=1.5), u.clamp(-1.5, 1.5) + 1
+        f = g * torch.sigmoid(1.702 * g)
+    else:
+        f = torch.nn.functional.silu(g) if act == "silu" else torch.relu(g)
+    # the activations have slopes of at most 1.2 and |f| <= |g| (clamped: 1.2 |g|)
+    slack = 2.0 ** -8 * (f * u).abs() + 1.2 * (eg * u.abs() + eu * g.abs() + eg * eu) + 1e-6
+    assert bool(((out.double() - f * u).abs() <= slack).all())
 
 
 @pytest.mark.parametrize("M", [1, 8])
@@ -90,11 +125,11 @@ def test_clamped_unit_and_biases(ops, M, N, K, biased):
     out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
     ops.gemm_few(a, w, out, M, kind="clamped", bias=bias, limit=limit, alpha=alpha)
     # slopes: the gate's function of at most 1.1 in the range that is clamped above, the linear branch's factor of at most 2.5
-    slack = 2.0 ** -8 * ref.abs() + 3 * BOUND * (scale[:, :N] + scale[:, N:] * g.abs()) + 1e-6
+    slack = 2.0 ** -8 * ref.abs() + 3 * bound(K) * (scale[:, :N] + scale[:, N:] * g.abs()) + 1e-6
     assert bool(((out.double() - ref).abs() <= slack).all())
     rows = torch.empty(M, 2 * N, device=DEV)
     ops.gemm_few(a, w, rows, M, bias=bias)
-    assert bool(((rows.double() - z).abs() <= BOUND * (scale + 1)).all())
+    assert bool(((rows.double() - z).abs() <= bound(K) * (scale + 1)).all())
 
 
 def test_what_is_not_taken(ops):
