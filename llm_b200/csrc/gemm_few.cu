@@ -368,8 +368,9 @@ int encode_weights(CUtensorMap* out, const void* w, long long rows, int K, long 
   return r == CUDA_SUCCESS ? 0 : llmk_fail(-2, "cuTensorMapEncodeTiled failed with %d", (int)r);
 }
 
-// What must be left beside the rows, in boxes: 8 rows of 8,448 leave room for three, and the tcgen05 kernel's swapped mode is ahead then (a call of the
-// design with that width 21.50 ms against 21.58); 3 rows of 14,336 leave four, and a decode step takes 3,198 us against 3,253.
+// What must be left beside the rows, in boxes of 16 KB; a gain of K numbers is counted with the rows whether they are normed or not, so that one limit
+// holds for all forms.  Beyond it the tcgen05 kernel's swapped mode is ahead.  Replayed decode steps, that kernel / this one: 8 rows of 8,448 (3.2
+// boxes left) 581 / 590 us, 5 rows of 14,336 (1.3) 2,930 / 2,995, 4 rows (3.03) 2,913 / 2,917, 2 rows (6.5) 2,894 / 2,846.
 constexpr int FEW_SMEM = 227 * 1024, FEW_LEAST_STAGES = 4;
 // The most that is in flight, and how much of it is asked for before the rows, which wait behind that.  Decode steps of 1.1 B (1, 4, 8 rows), all of the
 // ring first: 64 KB 771, 795, 828 us; 100 KB 695, 712, 746; 140 KB 666, 690, 750; 200 KB 677, 719, 755 (649, 675, 738 with 140 KB once the rows

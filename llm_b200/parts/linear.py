@@ -24,8 +24,9 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, rows: int, 
            bias: torch.Tensor = None, cta_limit: int = 0):
     """out[:rows] = x[:rows] @ weight.T (+ bias, float32 [out features]); out may be float32 for
     bfloat16 inputs.  cta_limit > 0 keeps a product of few rows to so many CTAs (it then leaves SMs
-    to the kernel after it).  With a bias the product is summed into `out` and the bias added there by a
-    kernel of its own (the reference adds it in the product's epilogue, model/modules/Linear.h:12-34).
+    to the kernel after it).  With a bias the product is summed into `out`; the product of few rows
+    adds it to its sums (the reference adds it in the product's epilogue too, model/modules/Linear.h:12-34), elsewhere a kernel of its own
+    adds it there.
 
     With allow_partial the result may come back as an ops.PartialSum (a split-K product whose
     partial results are still to be summed) instead of in `out`: pass it straight to a kernel
@@ -64,9 +65,9 @@ def linear_add(x: torch.Tensor, weight: torch.Tensor, stream: ResidualStream, ro
 def linear_swiglu(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, rows: int, act: str = "silu") -> bool:
     """out[:rows] = act(x @ gate.T) * (x @ up.T) for weight = [gate; up] stacked along its rows and act silu or relu,
     with the activation applied in the product's epilogue.  Returns False, having done nothing,
-    where that is not possible (float32, shapes the tensor-core kernel refuses, or so few rows
-    that the product splits its K dimension): the caller then runs the product and the activation
-    kernel."""
+    where that is not possible (float32, shapes that neither the product of few rows (up to 8) nor the one of
+    many (from 129) takes, 9 to 128 rows, whose product splits its K dimension): the caller then runs the product
+    and the activation kernel."""
     if rows == 0:
         return True
     if act in ("silu", "relu") and ops.gemm_few_available(x, weight, rows, gated=True):
@@ -83,8 +84,8 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, rows
 def linear_act(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, rows: int, act: str, bias: torch.Tensor = None) -> bool:
     """out[:rows] = act(x @ weight.T (+ bias, float32 [out features])) with the element-wise activation ("relu2", "gelu", "gelu_tanh", "silu")
     applied in the product's epilogue.  Returns False, having done nothing, where that is not possible
-    (float32, shapes the tensor-core kernel refuses, or so few rows that the product splits its K
-    dimension): the caller then runs the product and the activation kernel."""
+    (float32, shapes the tensor-core kernel refuses, or up to 128 rows, whose product splits its K dimension; the product of
+    few rows has no such epilogue): the caller then runs the product and the activation kernel."""
     if rows == 0:
         return True
     if act not in ops.EPILOGUE_ACTIVATIONS:
