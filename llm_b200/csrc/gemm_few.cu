@@ -363,8 +363,14 @@ int encode_weights(CUtensorMap* out, const void* w, long long rows, int K, long 
   if (!fn) return llmk_fail(-2, "cuTensorMapEncodeTiled is not available from the driver");
   cuuint64_t dims[3] = {(cuuint64_t)FEW_BLOCK, (cuuint64_t)rows, (cuuint64_t)(K / FEW_BLOCK)}, strides[2] = {(cuuint64_t)ldw * 2, FEW_BLOCK * 2};
   cuuint32_t box[3] = {FEW_BLOCK, (cuuint32_t)tile, (cuuint32_t)blocks}, step[3] = {1, 1, 1};
-  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(w), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto encode = [&] {
+    return fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(w), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  // a thread whose first call into CUDA this is: the runtime binds the device's context at its own calls, the driver's function does not
+  int device = 0;
+  if (r == CUDA_ERROR_INVALID_CONTEXT && cudaGetDevice(&device) == cudaSuccess && cudaSetDevice(device) == cudaSuccess) r = encode();
   return r == CUDA_SUCCESS ? 0 : llmk_fail(-2, "cuTensorMapEncodeTiled failed with %d", (int)r);
 }
 

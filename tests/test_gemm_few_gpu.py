@@ -145,7 +145,8 @@ def test_what_is_not_taken(ops):
 
 
 def test_two_threads_with_products_of_different_sizes(ops):
-    """Each launch takes the shared memory that its rows and stages need, whatever another thread launches at the same time."""
+    """Each launch takes the shared memory that its rows and stages need, whatever another thread launches at the same time; a product may be a
+    thread's first call into CUDA."""
     import threading
     small, large = operands(1, 96, 64), operands(8, 2368, 5632)
     want = [ops.gemm_few(a, w, torch.empty(a.shape[0], w.shape[0], device=DEV), a.shape[0]) for a, w in (small, large)]
