@@ -37,6 +37,8 @@ constexpr int PREFETCH_TILES = 4;      // tiles of keys and values that a warp a
 // float32, head size 32, one warp a head without parts / four warps / one warp with parts: 4,096 pairs of 8 keys 6.8 / 18.1 / 6.0, of 32 keys
 // 15.5 / 22.3 / 10.9, of 113 keys 47 / 36 / 34, of 1,000 keys 557 / 226 / 238; 2,048 pairs of 8 keys 6.0 / 10.1 / 5.0, of 32 keys 13.2 / 12.2 /
 // 8.0, of 113 keys 42 / 20 / 24, of 1,000 keys 353 / 126 / 171: up to 16 an SM what long contexts gain is more than what the shortest lose.
+// Beyond it one long prompt is what pays: 2,048 tokens, 4 heads of 32: 1,038 / 458 / 508 (551 before its last tokens, which have the most keys, came
+// first), 16 heads 3,356 / 1,667 / 1,727.
 constexpr int SERIAL_FROM = 16;
 __host__ __device__ constexpr int split_of(int max_dim) { return max_dim <= 64 ? WARPS : 1; }
 
@@ -103,8 +105,9 @@ paged_attention_generic_kernel(T* __restrict__ out, long long out_stride, const 
   pdl_launch_dependents();      // let the next kernel start its own prologue now
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long item = ((long long)blockIdx.x * WARPS + warp) / SHARE;
-  if (item >= (long long)n_tokens * n_heads) return;
+  const long long items = (long long)n_tokens * n_heads, place = ((long long)blockIdx.x * WARPS + warp) / SHARE;
+  if (place >= items) return;
+  const long long item = SERIAL ? items - 1 - place : place;      // the tokens with the most keys first, so that none of them ends alone
   const int t = (int)(item / n_heads), h = (int)(item % n_heads);
   const int g = h / (n_heads / n_kv);
   const int pos = positions[t];
@@ -141,8 +144,9 @@ paged_attention_generic_kernel(T* __restrict__ out, long long out_stride, const 
   float acc[MAXD / 32], m, l;
   __shared__ float m_s[WARPS / SHARE][SPLIT], l_s[WARPS / SHARE][SPLIT], acc_s[SPLIT > 1 ? WARPS / SHARE : 1][SPLIT][SPLIT > 1 ? MAXD : 1];
   const int owner = warp / SHARE;                  // of the (token, head) among the block's
+  int part = warp % SHARE;
 #pragma unroll 1
-  for (int part = warp % SHARE; part < used; part += SHARE) {
+  do {
 #pragma unroll
     for (int i = 0; i < MAXD / 32; ++i) acc[i] = 0.f;
     // the sink is the first term of the softmax: score 0, weight exp(0 - m), no value
@@ -210,7 +214,7 @@ paged_attention_generic_kernel(T* __restrict__ out, long long out_stride, const 
 #pragma unroll
       for (int i = 0; i < MAXD / 32; ++i) acc_s[owner][part][lane + 32 * i] = acc[i];
     }
-  }
+  } while (SERIAL && ++part < used);
   if (SPLIT > 1) {
     // the parts' sums in their order, against the largest of their maxima (a part without a tile, or with scores of -inf alone: -inf, weight
     // 0).  The values of a part of weight 0 are left out, as those of a key of weight 0 are: an infinite one would make a NaN.
