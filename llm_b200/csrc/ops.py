@@ -2021,15 +2021,16 @@ def gemm_few_takes(rows: int, k: int) -> bool:
 
 
 @functools.lru_cache(maxsize=4096)
-def gemm_few_pays(n: int, k: int, fused: bool, sms: int) -> bool:
+def gemm_few_pays(n: int, k: int, saves: int, sms: int) -> bool:
     """Whether n weight rows of k channels are few enough tiles for the few-row product.  A CTA walks over its tiles of 16 weight rows at 0.5 us each
-    at least, so that short rows on many tiles are better off on the tcgen05 kernel; fused: the product also saves a launch (a norm before it or
-    a gated activation behind it), which is worth four tiles.  Both sides, us a launch, tcgen05 / few-row: k 64, n 4,096 (two tiles a CTA) 2.0 /
+    at least, so that short rows on many tiles are better off on the tcgen05 kernel; saves: the tiles that the launch is worth which the product
+    saves, four for a gated activation behind it, two for a norm before it.  Both sides, us a launch, tcgen05 / few-row: k 64, n 4,096 (two tiles a CTA) 2.0 /
     2.2, 32,000 (14) 2.7 / 8.4; k 256, n 4,096 2.7 / 2.2, 6,144 2.8 / 2.9, 8,192 2.9 / 3.5; k 512, n 8,192 (4) 3.9 / 3.7, 16,384 (7) 4.6 / 5.4, 32,000
     6.8 / 9.0; k 768, n 16,384 6.4 / 5.9, 32,000 9.2 / 9.8; k 1,024, n 32,000 12.0 / 11.8, 128,256 (55) 51 / 40.  With the gated activation: k 64, n
-    8,192 4.0 / 3.5, 16,384 4.1 / 5.2; k 512, n 16,384 6.3 / 5.9, 32,000 8.5 / 10.0; k 768, n 32,000 11.1 / 10.6."""
+    8,192 4.0 / 3.5, 16,384 4.1 / 5.2; k 512, n 16,384 6.3 / 5.9, 32,000 8.5 / 10.0; k 768, n 32,000 11.1 / 10.6.  With the norm: k 64, n 8,192 3.3 / 3.6; k 128, n 8,192 3.5 / 3.6; k 256, n 8,192
+    4.0 / 3.7, 11,264 (5) 4.2 / 4.2, 16,384 4.3 / 5.3; k 512, n 16,384 5.9 / 5.5, 32,000 7.7 / 9.2; k 768, n 32,000 10.3 / 9.9."""
     tiles = _ceil_div(n, 16 * sms)
-    return k >= (768 if fused else 1024) or tiles <= max(1, k // 96) + (4 if fused else 0)
+    return k >= (768 if saves else 1024) or tiles <= max(1, k // 96) + saves
 
 
 def gemm_few_available(a, w: torch.Tensor, rows: int, gated: bool = False) -> bool:
@@ -2037,7 +2038,7 @@ def gemm_few_available(a, w: torch.Tensor, rows: int, gated: bool = False) -> bo
     with two halves of w."""
     if not GEMM_FEW or w.dtype != torch.bfloat16 or not gemm_few_takes(rows, w.shape[1]) or w.stride(0) % 8 or w.data_ptr() % 16 or not w.is_cuda:
         return False
-    if not gemm_few_pays(w.shape[0], w.shape[1], gated or isinstance(a, NormedRows), sm_count()):
+    if not gemm_few_pays(w.shape[0], w.shape[1], 4 if gated else 2 if isinstance(a, NormedRows) else 0, sm_count()):
         return False
     if isinstance(a, NormedRows):
         return a.resid.stride(0) % 4 == 0 and a.resid.data_ptr() % 16 == 0 and a.gain.data_ptr() % 16 == 0

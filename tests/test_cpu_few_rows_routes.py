@@ -42,18 +42,20 @@ def test_results_beyond_the_scratch_buffer_are_written_out(rows, n, unsummed, mo
     assert isinstance(got, ops.PartialSum) if unsummed else got is out
 
 
-@pytest.mark.parametrize("n,k,plain,fused", [(2368, 64, True, True), (2369, 64, False, True), (11840, 64, False, True), (11841, 64, False, False),
-                                             (4736, 256, True, True), (4737, 256, False, True), (11840, 512, True, True), (21312, 512, False, True),
-                                             (21313, 512, False, False), (32000, 512, False, False), (32000, 768, False, True), (32000, 1024, True, True),
-                                             (128256, 1024, True, True), (128256, 4096, True, True)])
-def test_short_rows_on_many_tiles_take_the_other_kernel(n, k, plain, fused, monkeypatch):
+@pytest.mark.parametrize("n,k,plain,normed,gated", [
+    (2368, 64, True, True, True), (2369, 64, False, True, True), (7104, 64, False, True, True), (7105, 64, False, False, True),
+    (11840, 64, False, False, True), (11841, 64, False, False, False), (4736, 256, True, True, True), (4737, 256, False, True, True),
+    (11840, 512, True, True, True), (16576, 512, False, True, True), (16577, 512, False, False, True), (21313, 512, False, False, False),
+    (32000, 768, False, True, True), (32000, 1024, True, True, True), (128256, 1024, True, True, True), (128256, 4096, True, True, True)])
+def test_short_rows_on_many_tiles_take_the_other_kernel(n, k, plain, normed, gated, monkeypatch):
     from llm_b200.csrc import ops
     monkeypatch.setattr(ops, "sm_count", lambda: 148)
     rows = torch.zeros(4, k, dtype=torch.bfloat16)
     a = types.SimpleNamespace(dtype=torch.bfloat16, is_cuda=True, stride=rows.stride, data_ptr=lambda: 0)
-    normed = ops.NormedRows(at(0, 4, k), at(0, k), 1e-5, 4, torch.bfloat16)
+    rows_under = ops.NormedRows(at(0, 4, k), at(0, k), 1e-5, 4, torch.bfloat16)
     assert ops.gemm_few_available(a, weights(n, k), 4) == plain
-    assert ops.gemm_few_available(a, weights(n, k), 4, gated=True) == ops.gemm_few_available(normed, weights(n, k), 4) == fused
+    assert ops.gemm_few_available(rows_under, weights(n, k), 4) == normed
+    assert ops.gemm_few_available(a, weights(n, k), 4, gated=True) == ops.gemm_few_available(rows_under, weights(n, k), 4, gated=True) == gated
 
 
 @pytest.mark.parametrize("rows,k,want", [(8, 4032, "few"), (8, 4096, "split"), (5, 6528, "few"), (5, 6592, "split"), (1, 14336, "few")])
