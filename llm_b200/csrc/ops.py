@@ -67,6 +67,7 @@ class NormedRows:
 
     def __init__(self, resid: torch.Tensor, gain: torch.Tensor, eps: float, rows: int, dtype: torch.dtype):
         self.resid, self.gain, self.eps, self.rows, self.dtype = resid, gain, eps, rows, dtype
+        self.aligned = resid.stride(0) % 4 == 0 and (resid.data_ptr() | gain.data_ptr()) % 16 == 0      # as the product copies them
 
 
 def _split_args(x):
@@ -2036,12 +2037,13 @@ def gemm_few_pays(n: int, k: int, saves: int, sms: int) -> bool:
 def gemm_few_available(a, w: torch.Tensor, rows: int, gated: bool = False) -> bool:
     """Whether gemm_few takes these operands, and is the faster one: bfloat16 (or NormedRows), few rows, 16-byte aligned.  gated: one of the kinds
     with two halves of w."""
-    if not GEMM_FEW or w.dtype != torch.bfloat16 or not gemm_few_takes(rows, w.shape[1]) or w.stride(0) % 8 or w.data_ptr() % 16 or not w.is_cuda:
+    n, k = w.shape
+    if not GEMM_FEW or w.dtype != torch.bfloat16 or not gemm_few_takes(rows, k) or w.stride(0) % 8 or w.data_ptr() % 16 or not w.is_cuda:
         return False
-    if not gemm_few_pays(w.shape[0], w.shape[1], 4 if gated else 2 if isinstance(a, NormedRows) else 0, sm_count()):
+    if k < 1024 and not gemm_few_pays(n, k, 4 if gated else 2 if isinstance(a, NormedRows) else 0, sm_count()):
         return False
     if isinstance(a, NormedRows):
-        return a.resid.stride(0) % 4 == 0 and a.resid.data_ptr() % 16 == 0 and a.gain.data_ptr() % 16 == 0
+        return a.aligned
     return a.dtype == torch.bfloat16 and a.is_cuda and a.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0
 
 
